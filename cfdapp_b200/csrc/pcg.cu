@@ -13,6 +13,10 @@
 // the device with no host round trip (the reference synchronises and sums on
 // the host once per reduction, DeviceVectorOpsKernel.cu:226-260).
 //
+// Systems that fit the chip's shared memory (up to 128^3) take the on-chip
+// form of the same method instead (resident.cuh); the streaming kernels here
+// serve the larger ones and the FP32-refined solves.
+//
 // The FP32-refined method runs the same kernel in FP32 (FP64 reductions)
 // inside FP64 iterative refinement: r = b - A x in FP64 (fused with the update
 // x += e), inner PCG on A e = r in FP32 to a moderate reduction, repeat until
@@ -605,7 +609,8 @@ double pcg_mixed_bytes(const cfdb_poperator* op, int64_t iterations, int64_t rep
   return init + per_it * (double)iterations + per_repl * (double)replacements;
 }
 
-// Algorithmic bytes of one persistent PCG launch: the initial pass reads b
+// Algorithmic bytes of one persistent PCG launch (the words its sweeps read
+// and write, wherever the vectors live): the initial pass reads b
 // (and x0) and writes r; each iteration moves 8 vector words per cell (sweep
 // A: r, p_old in, p out; sweep B: x, r, p in, x, r out) plus, with per-face
 // coefficients, the face words each sweep reads.  The TMA kernel also writes
@@ -712,14 +717,23 @@ cfdb_status solve_fp64(cfdb_context* ctx, cfdb_poperator* op, const cfdb_linear_
                        const double* b, double* x, bool x0_zero, int64_t hist_cap,
                        cfdb_linear_result* res) {
   const int64_t n = op->cells;
+  // on chip where it fits: the exchanged values (w64[1]) and the inverse
+  // diagonal of a table operator (w64[6]) are its only vectors in memory
+  const bool chip = resident_pcg_fits(ctx, view<double>(op));
   for (int q : {0, 1, 2, 6}) {
+    if (chip && q != 1 && (q != 6 || op->invd64)) continue;
     cfdb_status st = alloc_vec(ctx, &op->w64[q], n);
     if (st != CFDB_OK) return st;
   }
   cfdb_status st = ensure_hist(ctx, op, std::max<int64_t>(hist_cap, 1));
   if (st != CFDB_OK) return st;
-  st = run_pcg<double>(ctx, op, b, x, op->w64[0], op->w64[1], op->w64[2], op->w64[6], x0_zero ? 1 : 0,
-                       s->abs_tol, s->rel_tol, s->max_iterations, op->hist_dev, hist_cap);
+  if (chip)
+    st = resident_pcg(ctx, view<double>(op), op->grid.dim, op->invd64, b, x, op->w64[1],
+                      op->invd64 ? nullptr : op->w64[6], s->abs_tol, s->rel_tol,
+                      s->max_iterations, op->hist_dev, hist_cap);
+  else
+    st = run_pcg<double>(ctx, op, b, x, op->w64[0], op->w64[1], op->w64[2], op->w64[6], x0_zero ? 1 : 0,
+                         s->abs_tol, s->rel_tol, s->max_iterations, op->hist_dev, hist_cap);
   if (st != CFDB_OK) return st;
   st = read_scalars(ctx, 8);
   if (st != CFDB_OK) return st;

@@ -4,6 +4,7 @@
 #include <cstdint>
 
 #include "cfdb.h"
+#include "poperator.cuh"
 
 namespace cfdb {
 struct LearnedSolver;
@@ -13,4 +14,13 @@ cfdb_status poperator_bind_faces(cfdb_context* ctx, cfdb_poperator* op, const do
 // (created on first use) and coefficient version.
 void poperator_learned(cfdb_poperator* op, FineOperator* fo, LearnedSolver** solver,
                        uint64_t* version);
+// The on-chip FP64 Jacobi-PCG (resident_faces.cu): whether a system
+// fits, and the solve (x in and out; `pub`, `inv`: vectors of `cells`,
+// inv null where invd is given).  The
+// outcome lands in the context's scalars.
+bool resident_pcg_fits(const cfdb_context* ctx, const OpView<double>& A);
+cfdb_status resident_pcg(cfdb_context* ctx, const OpView<double>& A, int dim, const double* invd,
+                         const double* b, double* x, double* pub, double* inv,
+                         double abs_tol, double rel_tol,
+                         int64_t max_it, double* hist, int64_t hist_cap);
 }

@@ -1,0 +1,661 @@
+// Krylov solves whose vectors stay on chip.
+//
+// The streaming solvers (pcg_tma.cuh, stencil_krylov.cuh) move every vector
+// through L2 once or more per iteration and cross the whole GPU in grid
+// barriers built on one atomic counter.  A system that fits the chip needs
+// neither: here every block owns one contiguous range of cells for the whole
+// solve, keeps the vectors of its cells in shared memory and registers, and
+// an iteration only exchanges the values of p at the ends of the ranges and
+// the partial sums of the dot products.  What is left is the latency of the
+// dependent steps: p -> A p -> alpha -> r -> beta.
+//
+// Two teams of blocks run the same routines:
+//   ClusterTeam  one thread-block cluster of 1..16 blocks.  Neighbours read
+//                each other's values in distributed shared memory, partial sums
+//                are pushed into every block's shared memory, and the barrier is
+//                the hardware cluster barrier.
+//   GridTeam     one block per SM, cooperatively launched.  Values are
+//                published in global memory (L2); a reduction is one release-
+//                add on a counter and one acquiring poll (bounded) by one thread
+//                per block, then every block adds all partial sums: 2.2 us with
+//                148 blocks of 512 threads (an all-to-all exchange of tagged
+//                values, polled without a counter, took 3.7 to 5.5 us for two
+//                values: the polls contend with the writes).
+//
+// All sums run in a fixed order (threads by shuffle, warps, then blocks by
+// rank), so a result does not depend on timing, and every block derives
+// bitwise-identical scalars and takes the same branch.
+#pragma once
+
+#include <cuda_runtime.h>
+
+#include <cfloat>
+#include <cmath>
+#include <cstdint>
+
+#include "cfdb.h"
+#include "grid_sync.cuh"
+#include "poperator.cuh"
+#include "stencil_solve.cuh"
+
+namespace cfdb {
+namespace res {
+
+// Division of a cell index (< 2^31) by a fixed divisor: one 32 x 32 -> 64
+// multiply (m = ceil(2^s / d), s = 31 + ceil(log2 d), m < 2^32).
+struct FastDiv {
+  uint32_t m = 0, s = 31;
+  __device__ __forceinline__ uint32_t div(uint32_t c) const {
+    return (uint32_t)(((uint64_t)c * m) >> s);
+  }
+};
+inline FastDiv fast_div(uint32_t d) {
+  FastDiv f;
+  uint32_t l = 0;
+  while ((1ull << l) < d) ++l;
+  f.s = 31 + l;
+  f.m = (uint32_t)(((1ull << f.s) + d - 1) / d);
+  return f;
+}
+
+// Couplings of one cell to its neighbours (0 across the domain's edge), its
+// diagonal and the preconditioner's inverse diagonal.
+struct Cf {
+  double xl, xh, yl, yh, zl, zh, dg, inv;
+};
+
+// ------------------------------------------------------------------ operators
+//
+// An operator has the extents of kernel space (a 2D grid is nx x 1 x ny),
+// load() -> Cf of a cell and mul() -> the row's product.
+
+// The p' operator (poperator.cuh), tables or face arrays; Jacobi.
+template <int DIM>
+struct FaceOp {
+  static constexpr int kDim = DIM;
+  OpView<double> A;
+  const double* invd;  // 1/diag of face-array operators, or null
+  int nx, ny, nz;
+  uint32_t sz;
+  FastDiv dx, dy;
+  __device__ __forceinline__ Cf load(uint32_t c, int i, int j, int k) const {
+    Cf f;
+    const uint32_t row = (uint32_t)j + (uint32_t)ny * k;
+    if (A.fx) {
+      f.xl = __ldg(A.fx + c + row);
+      f.xh = __ldg(A.fx + c + row + 1);
+    } else {
+      f.xl = __ldg(A.tx + i);
+      f.xh = __ldg(A.tx + i + 1);
+    }
+    f.yl = f.yh = 0.0;
+    if (DIM == 3) {
+      if (A.fy) {
+        f.yl = __ldg(A.fy + c + (uint32_t)nx * k);
+        f.yh = __ldg(A.fy + c + (uint32_t)nx * k + nx);
+      } else {
+        f.yl = __ldg(A.ty + j);
+        f.yh = __ldg(A.ty + j + 1);
+      }
+    }
+    if (A.fz) {
+      f.zl = __ldg(A.fz + c);
+      f.zh = __ldg(A.fz + c + sz);
+    } else {
+      f.zl = __ldg(A.tz + k);
+      f.zh = __ldg(A.tz + k + 1);
+    }
+    if (A.pinned && c == (uint32_t)A.ref) {
+      f.xl = f.xh = f.yl = f.yh = f.zl = f.zh = 0.0;
+      f.dg = f.inv = 1.0;
+      return f;
+    }
+    // the reference's face order (poperator.cuh load_coef)
+    f.dg = ((((f.xl + f.xh) + f.yl) + f.yh) + f.zl) + f.zh;
+    f.inv = invd ? __ldg(invd + c) : rcp_rn(f.dg);
+    if (i == 0) f.xl = 0.0;
+    if (i == nx - 1) f.xh = 0.0;
+    if (j == 0) f.yl = 0.0;
+    if (j == ny - 1) f.yh = 0.0;
+    if (k == 0) f.zl = 0.0;
+    if (k == nz - 1) f.zh = 0.0;
+    return f;
+  }
+  // the preconditioner's inverse diagonal alone
+  __device__ __forceinline__ double inverse(uint32_t c, int i, int j, int k) const {
+    if (invd) return __ldg(invd + c);
+    if (A.fx || A.fy || A.fz) return load(c, i, j, k).inv;
+    if (A.pinned && c == (uint32_t)A.ref) return 1.0;
+    double d = __ldg(A.tx + i) + __ldg(A.tx + i + 1);
+    if (DIM == 3) d = (d + __ldg(A.ty + j)) + __ldg(A.ty + j + 1);
+    return rcp_rn((d + __ldg(A.tz + k)) + __ldg(A.tz + k + 1));
+  }
+  __device__ __forceinline__ double mul(const Cf& f, double v, double w, double e, double s,
+                                        double n, double b, double t) const {
+    double off = f.xl * w;
+    off = fma(f.xh, e, off);
+    if (DIM == 3) {
+      off = fma(f.yl, s, off);
+      off = fma(f.yh, n, off);
+    }
+    off = fma(f.zl, b, off);
+    off = fma(f.zh, t, off);
+    return fma(f.dg, v, -off);
+  }
+};
+
+// A stored stencil matrix (stencil_solve.cuh); inv null: no preconditioner.
+// A 2D matrix's second axis is kernel space's z.
+template <int DIM>
+struct BandOp {
+  static constexpr int kDim = DIM;
+  const double* diag;
+  const double *oxl, *oxh, *oyl, *oyh, *ozl, *ozh;
+  const double* pinv;
+  int nx, ny, nz;
+  uint32_t sz;
+  FastDiv dx, dy;
+  __device__ __forceinline__ Cf load(uint32_t c, int i, int j, int k) const {
+    Cf f;
+    f.xl = i > 0 ? __ldg(oxl + c) : 0.0;
+    f.xh = i < nx - 1 ? __ldg(oxh + c) : 0.0;
+    f.yl = DIM == 3 && j > 0 ? __ldg(oyl + c) : 0.0;
+    f.yh = DIM == 3 && j < ny - 1 ? __ldg(oyh + c) : 0.0;
+    f.zl = k > 0 ? __ldg(ozl + c) : 0.0;
+    f.zh = k < nz - 1 ? __ldg(ozh + c) : 0.0;
+    f.dg = __ldg(diag + c);
+    f.inv = pinv ? __ldg(pinv + c) : 1.0;
+    return f;
+  }
+  __device__ __forceinline__ double inverse(uint32_t c, int, int, int) const {
+    return pinv ? __ldg(pinv + c) : 1.0;
+  }
+  // ascending column order of the reference's CSR rows
+  __device__ __forceinline__ double mul(const Cf& f, double v, double w, double e, double s,
+                                        double n, double b, double t) const {
+    double sum = f.zl * b;
+    if (DIM == 3) sum += f.yl * s;
+    sum += f.xl * w;
+    sum += f.dg * v;
+    sum += f.xh * e;
+    if (DIM == 3) sum += f.yh * n;
+    sum += f.zh * t;
+    return sum;
+  }
+};
+
+template <int DIM>
+BandOp<DIM> band_op(const StencilMatrix& M) {
+  BandOp<DIM> A{};
+  A.diag = M.diag;
+  A.oxl = M.off[0];
+  A.oxh = M.off[1];
+  if (DIM == 3) {
+    A.oyl = M.off[2];
+    A.oyh = M.off[3];
+    A.ozl = M.off[4];
+    A.ozh = M.off[5];
+  } else {
+    A.ozl = M.off[2];
+    A.ozh = M.off[3];
+  }
+  A.pinv = M.inv;
+  A.nx = M.nx;
+  A.ny = DIM == 3 ? M.ny : 1;
+  A.nz = DIM == 3 ? M.nz : M.ny;
+  A.sz = (uint32_t)A.nx * A.ny;
+  A.dx = fast_div(A.nx);
+  A.dy = fast_div(A.ny);
+  return A;
+}
+
+// ---------------------------------------------------------------------- teams
+
+constexpr int kMaxCluster = 16;
+constexpr int kMaxVals = 3;
+
+// Sum of N values of an array by halves (fixed order; N a power of two).
+template <int N>
+__device__ __forceinline__ double tree(double (&a)[N]) {
+#pragma unroll
+  for (int w = N / 2; w > 0; w >>= 1)
+#pragma unroll
+    for (int s = 0; s < w; ++s) a[s] += a[s + w];
+  return a[0];
+}
+
+// Block-wide sum in a fixed order, valid in every thread of warp 0 (`W`
+// warps, a power of two).  The warps' sums are added from shared memory by a
+// tree in registers: half the latency of a second round of shuffles.
+template <int NV, int W>
+__device__ __forceinline__ void block_total(double (&v)[NV], double (*red)[32]) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+  for (int q = 0; q < NV; ++q)
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) v[q] += __shfl_xor_sync(0xffffffffu, v[q], off);
+  if (lane == 0)
+#pragma unroll
+    for (int q = 0; q < NV; ++q) red[q][warp] = v[q];
+  __syncthreads();
+  if (warp == 0) {
+#pragma unroll
+    for (int q = 0; q < NV; ++q) {
+      double a[W];
+#pragma unroll
+      for (int s = 0; s < W; ++s) a[s] = red[q][s];
+      v[q] = tree<W>(a);
+    }
+  }
+}
+
+struct TeamSmem {
+  alignas(16) double red[kMaxVals][32];
+  alignas(16) double slot[2][kMaxVals][kMaxCluster];  // cluster: every block's sums, by parity
+  alignas(16) double poll[kMaxVals][8];               // grid: the polling warps' sums
+};
+
+template <int T>
+struct ClusterTeam {
+  static constexpr bool kGlobal = false;
+  int rank_, size_;
+  int parity = 0;
+  FastDiv dlen;
+  uint32_t len;
+  TeamSmem* ts;
+  __device__ int rank() const { return rank_; }
+  __device__ __forceinline__ bool sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;"
+                 ::: "memory");
+    return true;
+  }
+  // The team-wide sums of v, in every thread; a full barrier of the team.
+  template <int NV>
+  __device__ __forceinline__ bool reduce(double (&v)[NV]) {
+    block_total<NV, T / 32>(v, ts->red);
+    if ((int)threadIdx.x < size_) {
+#pragma unroll
+      for (int q = 0; q < NV; ++q) {
+        const uint32_t a = (uint32_t)__cvta_generic_to_shared(&ts->slot[parity][q][rank_]);
+        uint32_t ra;
+        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(a), "r"(threadIdx.x));
+        asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(ra), "d"(v[q]) : "memory");
+      }
+    }
+    sync();
+#pragma unroll
+    for (int q = 0; q < NV; ++q) {
+      double a[kMaxCluster];
+#pragma unroll
+      for (int s = 0; s < kMaxCluster; ++s) a[s] = s < size_ ? ts->slot[parity][q][s] : 0.0;
+      v[q] = tree<kMaxCluster>(a);
+    }
+    parity ^= 1;
+    return true;
+  }
+  // vec[c] of a cell outside this block's range (vec: this block's shared array)
+  __device__ __forceinline__ double remote(const double* vec, const double*, uint32_t c) const {
+    const uint32_t r = dlen.div(c);
+    const uint32_t a = (uint32_t)__cvta_generic_to_shared(vec + (c - r * len));
+    uint32_t ra;
+    double out;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(a), "r"(r));
+    asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(out) : "r"(ra) : "memory");
+    return out;
+  }
+};
+
+template <int T>
+struct GridTeam {
+  static constexpr bool kGlobal = true;
+  static constexpr int kPollers = 256;  // threads that read the partial sums: >= blocks
+  static_assert(T >= kPollers, "one thread per block reads its partial sums");
+  double* partials;  // 2 parities x blocks x kMaxVals
+  unsigned* count;   // arrivals since the launch (wraps)
+  unsigned* error;
+  unsigned long long timeout_ns;
+  int rank_, size_;
+  unsigned round = 0;
+  TeamSmem* ts;
+  __device__ int rank() const { return rank_; }
+  // Thread 0 arrives (after a block barrier: its release covers the whole
+  // block's stores) and waits, bounded, for every block of this round.
+  __device__ __forceinline__ bool arrive_and_wait() {
+    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(count) : "memory");
+    const unsigned target = round * (unsigned)size_;
+    unsigned long long t0 = 0;
+    for (unsigned spin = 0;; ++spin) {
+      unsigned c;
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(c) : "l"(count) : "memory");
+      if ((int)(c - target) >= 0) return *(volatile unsigned*)error == 0u;
+      if ((spin & 63u) != 63u) continue;
+      const unsigned long long now = global_ns();
+      if (t0 == 0) t0 = now;
+      if (*(volatile unsigned*)error != 0u) return false;
+      if (now - t0 > timeout_ns) {
+        atomicExch(error, 1u);
+        return false;
+      }
+    }
+  }
+  // published values are visible to every block afterwards
+  __device__ __forceinline__ bool sync() {
+    ++round;
+    __syncthreads();
+    bool ok = true;
+    if (threadIdx.x == 0) ok = arrive_and_wait();
+    return __syncthreads_and(ok);
+  }
+  // The team-wide sums of v, in every thread; a full barrier of the team.
+  template <int NV>
+  __device__ __forceinline__ bool reduce(double (&v)[NV]) {
+    block_total<NV, T / 32>(v, ts->red);
+    ++round;
+    double* base = partials + (size_t)(round & 1) * size_ * kMaxVals;
+    const int t = threadIdx.x;
+    bool ok = true;
+    if (t == 0) {
+#pragma unroll
+      for (int q = 0; q < NV; ++q) __stcg(base + rank_ * NV + q, v[q]);
+      ok = arrive_and_wait();
+    }
+    if (!__syncthreads_and(ok)) return false;
+    if (t < kPollers) {
+      double a[NV];
+#pragma unroll
+      for (int q = 0; q < NV; ++q) a[q] = t < size_ ? __ldcg(base + t * NV + q) : 0.0;
+#pragma unroll
+      for (int q = 0; q < NV; ++q)
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) a[q] += __shfl_xor_sync(0xffffffffu, a[q], off);
+      if ((t & 31) == 0)
+#pragma unroll
+        for (int q = 0; q < NV; ++q) ts->poll[q][t >> 5] = a[q];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < NV; ++q) {
+      double b[kPollers / 32];
+#pragma unroll
+      for (int s = 0; s < kPollers / 32; ++s) b[s] = ts->poll[q][s];
+      v[q] = tree<kPollers / 32>(b);
+    }
+    return true;
+  }
+  __device__ __forceinline__ double remote(const double*, const double* pub, uint32_t c) const {
+    return __ldcg(pub + c);
+  }
+};
+
+// ------------------------------------------------------------------- routines
+
+struct Io {
+  const double* b;
+  double* x;
+  double* pub;   // GridTeam: published values (cells), else null
+  double* inv;   // scratch (cells) for M^-1 of a table operator, or null
+  double abs_tol, rel_tol;
+  int64_t max_it;
+  double* hist;
+  int64_t hist_cap;
+  double* out;  // status, iterations, initial residual, final residual, restarts
+};
+
+// Range of cells of block `rank`: [rank len, min(n, (rank + 1) len)).
+struct Range {
+  uint32_t c0, count;
+};
+__device__ __forceinline__ Range range_of(uint32_t n, uint32_t len, int rank) {
+  const uint32_t c0 = min(n, len * (uint32_t)rank);
+  return Range{c0, min(len, n - c0)};
+}
+
+// The coefficients of a thread's NC cells: kept in registers for the whole
+// solve when there are few of them, else loaded again where they are used.
+template <class Op, int NC, bool PRE>
+struct Cells {
+  Cf f[PRE ? NC : 1];
+  __device__ __forceinline__ void ijk(const Op& A, uint32_t c, int& i, int& j, int& k) const {
+    const uint32_t row = A.dx.div(c);
+    i = (int)(c - row * (uint32_t)A.nx);
+    if (Op::kDim == 3) {
+      const uint32_t kk = A.dy.div(row);
+      k = (int)kk;
+      j = (int)(row - kk * (uint32_t)A.ny);
+    } else {
+      k = (int)row;
+      j = 0;
+    }
+  }
+  __device__ __forceinline__ Cf load(const Op& A, uint32_t c) const {
+    int i, j, k;
+    ijk(A, c, i, j, k);
+    return A.load(c, i, j, k);
+  }
+  template <int T>
+  __device__ __forceinline__ void init(const Op& A, const Range& R) {
+    if constexpr (PRE) {
+#pragma unroll
+      for (int q = 0; q < NC; ++q) {
+        const uint32_t lc = threadIdx.x + q * T;
+        if (lc < R.count) f[q] = load(A, R.c0 + lc);
+      }
+    }
+  }
+  __device__ __forceinline__ Cf at(const Op& A, int q, uint32_t c) const {
+    if constexpr (PRE) return f[q];
+    else return load(A, c);
+  }
+  __device__ __forceinline__ double inverse(const Op& A, int q, uint32_t c) const {
+    if constexpr (PRE) return f[q].inv;
+    int i, j, k;
+    ijk(A, c, i, j, k);
+    return A.inverse(c, i, j, k);
+  }
+};
+
+// (A v)(c) with v in this block's shared array.  HALO: every neighbour is in
+// the array.  Else x- and y-neighbours past the range's ends are read from
+// the published vector (couplings of 0 read nothing), and the z-neighbours'
+// values come with the call.
+template <bool HALO, class Op, class Team>
+__device__ __forceinline__ double apply(const Op& A, const Team& T, const Cf& f, const Range& R,
+                                        uint32_t lc, const double* vec, const double* pub,
+                                        double zlo, double zhi) {
+  const int sy = A.nx, sz = (int)A.sz;
+  const double* v = vec + lc;
+  if constexpr (HALO) {
+    return A.mul(f, v[0], v[-1], v[1], Op::kDim == 3 ? v[-sy] : 0.0, Op::kDim == 3 ? v[sy] : 0.0,
+                 v[-sz], v[sz]);
+  } else {
+    const uint32_t c = R.c0 + lc;
+    auto get = [&](double coupling, int off) -> double {
+      const uint32_t li = lc + (uint32_t)off;  // wraps below 0: past count
+      if (li < R.count) return vec[li];
+      return coupling == 0.0 ? 0.0 : T.remote(vec, pub, c + (uint32_t)off);
+    };
+    return A.mul(f, v[0], get(f.xl, -1), get(f.xh, 1), Op::kDim == 3 ? get(f.yl, -sy) : 0.0,
+                 Op::kDim == 3 ? get(f.yh, sy) : 0.0, zlo, zhi);
+  }
+}
+
+// (A x)(c) with x in global memory.
+template <class Op>
+__device__ __forceinline__ double apply_global(const Op& A, const Cf& f, uint32_t c,
+                                               const double* x) {
+  auto get = [&](double coupling, uint32_t at) { return coupling == 0.0 ? 0.0 : __ldcg(x + at); };
+  const uint32_t sy = (uint32_t)A.nx, sz = A.sz;
+  return A.mul(f, __ldcg(x + c), get(f.xl, c - 1), get(f.xh, c + 1),
+               Op::kDim == 3 ? get(f.yl, c - sy) : 0.0, Op::kDim == 3 ? get(f.yh, c + sy) : 0.0,
+               get(f.zl, c - sz), get(f.zh, c + sz));
+}
+
+// Jacobi-CG (or plain CG), the reference's method and tests (CG.cpp:14-148).
+//
+// HALO: the block also keeps p of the H = one plane (2D: row) of cells before
+// and after its range, and forms it there as its owners do, from the
+// published z = M^-1 r and its own old p; an iteration then has two exchanges
+// (the two reductions).  Otherwise (3D grids whose planes are larger than
+// shared memory allows) p itself is published, which takes a third.
+//
+// Shared memory (doubles): p (len, HALO: + 2 H), r (len), ClusterTeam: z
+// (len), XS: x (len).
+template <int T, int NC, bool PRE, bool XS, bool HALO, class Op, class Team>
+__device__ __forceinline__ void cg_run(const Op& A, uint32_t n, uint32_t len, const Io& P,
+                                       Team& team, double* sm) {
+  static_assert(HALO || Team::kGlobal, "a cluster's planes fit its shared memory");
+  const Range R = range_of(n, len, team.rank());
+  const uint32_t H = A.sz;  // reach of the stencil
+  double* p = HALO ? sm + H : sm;
+  double* r = sm + len + (HALO ? 2 * H : 0);
+  double* zs = r + len;
+  double* xs = zs + (Team::kGlobal ? 0 : len);
+  const bool leader = team.rank() == 0 && threadIdx.x == 0;
+  Cells<Op, NC, PRE> cells;
+  cells.template init<T>(A, R);
+  if (HALO)
+    for (uint32_t q = threadIdx.x; q < len + 2 * H; q += T) sm[q] = 0.0;
+  double z[NC];  // z = M^-1 r between the sweeps, q = A p within an iteration
+  // z of a cell for the blocks whose stencils reach it
+  auto publish = [&](uint32_t lc, double v) {
+    if (!Team::kGlobal) zs[lc] = v;
+    else if (!HALO || lc < H || lc + H >= R.count) P.pub[R.c0 + lc] = v;
+  };
+  double acc[2] = {0.0, 0.0};
+#pragma unroll
+  for (int q = 0; q < NC; ++q) {
+    const uint32_t lc = threadIdx.x + q * T;
+    if (lc < R.count) {
+      const uint32_t c = R.c0 + lc;
+      const Cf f = cells.at(A, q, c);
+      const double rn = __ldg(P.b + c) - apply_global(A, f, c, P.x);
+      r[lc] = rn;
+      if (XS) xs[lc] = __ldcg(P.x + c);
+      z[q] = f.inv * rn;
+      if (HALO) publish(lc, z[q]);
+      if (!PRE && P.inv) P.inv[c] = f.inv;
+      acc[0] += rn * rn;
+      acc[1] += rn * z[q];
+    }
+  }
+  if (!team.reduce(acc)) return;
+  const double b0 = sqrt(acc[0]);
+  double rz = acc[1];
+  auto conv = [&](double res) {
+    return (res <= P.abs_tol) || ((b0 > 0.0) && (res / b0 <= P.rel_tol));
+  };
+  auto finish = [&](int status, int64_t it, double fin) {
+    if (leader) {
+      P.out[0] = status;
+      P.out[1] = (double)it;
+      P.out[3] = fin;
+    }
+    if (XS && it > 0) {
+#pragma unroll
+      for (int q = 0; q < NC; ++q) {
+        const uint32_t lc = threadIdx.x + q * T;
+        if (lc < R.count) P.x[R.c0 + lc] = xs[lc];
+      }
+    }
+  };
+  if (leader) {
+    P.out[2] = b0;
+    P.out[4] = 0.0;
+    if (P.hist_cap > 0) P.hist[0] = b0;
+  }
+  if (b0 == 0.0 || conv(b0)) return finish(CFDB_SOLVER_CONVERGED, 0, b0);
+  if (!isfinite(rz)) return finish(CFDB_SOLVER_BREAKDOWN, 0, b0);
+  // cells of the halo inside the domain: [lo0, c0) and [c0 + count, hi1)
+  const uint32_t lo = min(H, R.c0), hi = min(H, n - (R.c0 + R.count));
+  double res_cur = b0, beta = 0.0;
+  for (int64_t it = 1; it <= P.max_it; ++it) {
+    // p = z + beta p
+    if (HALO && R.count > 0) {
+      for (uint32_t h = threadIdx.x; h < lo + hi; h += T) {
+        const int at = h < lo ? -(int)(lo - h) : (int)(R.count + (h - lo));
+        p[at] = fma(beta, p[at], team.remote(zs, P.pub, R.c0 + (uint32_t)at));
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < NC; ++q) {
+      const uint32_t lc = threadIdx.x + q * T;
+      if (lc < R.count) {
+        const double v = it == 1 ? z[q] : fma(beta, p[lc], z[q]);
+        p[lc] = v;
+        if (!HALO) publish(lc, v);
+      }
+    }
+    if (HALO) __syncthreads();
+    else if (!team.sync()) return;
+    double pap[1] = {0.0};
+    if constexpr (HALO) {
+#pragma unroll
+      for (int q = 0; q < NC; ++q) {
+        const uint32_t lc = threadIdx.x + q * T;
+        if (lc < R.count) {
+          const Cf f = cells.at(A, q, R.c0 + lc);
+          z[q] = apply<true>(A, team, f, R, lc, p, P.pub, 0.0, 0.0);
+          pap[0] += p[lc] * z[q];
+        }
+      }
+    } else {
+      // the z-neighbours of a batch of cells, all from L2, are loaded before
+      // the first is used
+      constexpr int G = NC % 4 == 0 ? 4 : (NC % 2 == 0 ? 2 : 1);
+#pragma unroll
+      for (int g = 0; g < NC; g += G) {
+        double lo_z[G], hi_z[G];
+#pragma unroll
+        for (int u = 0; u < G; ++u) {
+          const uint32_t c = R.c0 + threadIdx.x + (g + u) * T;
+          const bool in = threadIdx.x + (g + u) * T < R.count;
+          lo_z[u] = in && c >= H ? __ldcg(P.pub + (c - H)) : 0.0;
+          hi_z[u] = in && c + H < n ? __ldcg(P.pub + (c + H)) : 0.0;
+        }
+#pragma unroll
+        for (int u = 0; u < G; ++u) {
+          const int q = g + u;
+          const uint32_t lc = threadIdx.x + q * T;
+          if (lc < R.count) {
+            const Cf f = cells.at(A, q, R.c0 + lc);
+            z[q] = apply<false>(A, team, f, R, lc, p, P.pub, lo_z[u], hi_z[u]);
+            pap[0] += p[lc] * z[q];
+          }
+        }
+      }
+    }
+    if (!team.reduce(pap)) return;
+    const double pAp = pap[0];
+    const double alpha = rz / pAp;
+    if (!isfinite(pAp) || fabs(pAp) < 1.0e-30 || !isfinite(alpha))
+      return finish(CFDB_SOLVER_BREAKDOWN, it - 1, res_cur);
+    double ab[2] = {0.0, 0.0};
+#pragma unroll
+    for (int q = 0; q < NC; ++q) {
+      const uint32_t lc = threadIdx.x + q * T;
+      if (lc < R.count) {
+        if (XS) xs[lc] = fma(alpha, p[lc], xs[lc]);
+        else P.x[R.c0 + lc] = fma(alpha, p[lc], P.x[R.c0 + lc]);
+        const double rn = fma(-alpha, z[q], r[lc]);
+        r[lc] = rn;
+        z[q] = (!PRE && P.inv ? P.inv[R.c0 + lc] : cells.inverse(A, q, R.c0 + lc)) * rn;
+        if (HALO) publish(lc, z[q]);
+        ab[0] += rn * rn;
+        ab[1] += rn * z[q];
+      }
+    }
+    if (!team.reduce(ab)) return;
+    const double res = sqrt(ab[0]);
+    if (leader && it < P.hist_cap) P.hist[it] = res;
+    if (!isfinite(res)) return finish(CFDB_SOLVER_NONFINITE_RESIDUAL, it, res);
+    res_cur = res;
+    if (conv(res)) return finish(CFDB_SOLVER_CONVERGED, it, res);
+    beta = ab[1] / rz;
+    if (!isfinite(ab[1]) || !isfinite(beta)) return finish(CFDB_SOLVER_BREAKDOWN, it, res);
+    rz = ab[1];
+  }
+  finish(CFDB_SOLVER_MAX_ITERATIONS, P.max_it, res_cur);
+}
+
+}  // namespace res
+}  // namespace cfdb

@@ -1,0 +1,184 @@
+// Choice and launch of the on-chip Krylov kernels (resident.cuh).
+#pragma once
+
+#include <cuda_runtime.h>
+
+#include <algorithm>
+#include <map>
+#include <mutex>
+#include <utility>
+
+#include "cfdb_internal.cuh"
+#include "resident.cuh"
+
+namespace cfdb {
+namespace res {
+
+constexpr unsigned long long kTimeoutNs = 2000000000ull;
+constexpr size_t kSmemMax = 225 * 1024;  // of the 227 KB a block may have, beside TeamSmem
+constexpr int kClusterThreads = 512;
+constexpr int kClusterNC = 8, kGridNC = 14;  // most cells per thread
+// Threads of a grid team's blocks: 1024 once every thread has several cells
+// (a reduction over 512 threads is 0.5 us faster).
+constexpr int kGridThreadsSmall = 512, kGridThreadsLarge = 1024;
+constexpr uint32_t kGridSmallCells = 2048;  // cells per block
+
+struct Plan {
+  int team = 0;  // 0: does not fit; 1: one cluster; 2: the grid
+  int blocks = 0;
+  uint32_t len = 0;
+  int nc = 0;
+  bool xs = false;    // x in shared memory too
+  int threads = 0;
+  bool halo = false;  // p of the neighbouring planes kept in shared memory
+  size_t smem = 0;
+};
+
+// Cells a cluster takes before the whole GPU is the faster team, by the time
+// of a CG iteration (us, cluster / grid): 129^2 4.7 / 6.6, 181^2 (32 761 cells)
+// 5.6 / 6.6, 33^3 7.5 / 7.2, 250^2 8.0 / 6.7, 40^3 10.2 / 6.7.
+constexpr int64_t kClusterCells = 36864;
+
+// Layout of the CG of n cells.  A cluster's size grows with the system until every
+// block has one cell per thread; per iteration (us, streaming kernel before):
+// 40x33 2.7 (18.6), 129^2 4.7 (13.0), 512^2 8.0 (20.9), 64^3 9.6 (19.5),
+// 96^3 16.7 (29.3), 128^3 31.8 (44.7); the last two keep no neighbouring
+// planes.  `reach`: cells the stencil reaches (a plane).
+inline Plan cg_plan(int64_t n, int64_t reach, int num_sms, int max_cluster) {
+  Plan P;
+  auto fill = [&](int team, int blocks, int max_nc, bool halo) {
+    P = Plan{};
+    P.len = (uint32_t)((n + blocks - 1) / blocks);
+    const int threads = team == 1 ? kClusterThreads
+                                  : (P.len <= kGridSmallCells ? kGridThreadsSmall : kGridThreadsLarge);
+    P.threads = threads;
+    P.blocks = team == 1 ? blocks : (int)((n + P.len - 1) / P.len);
+    P.nc = (int)((P.len + threads - 1) / threads);
+    P.halo = halo;
+    const size_t words = (size_t)P.len * (team == 1 ? 3 : 2) + (halo ? 2 * (size_t)reach : 0);
+    P.xs = (words + P.len) * 8 <= kSmemMax;
+    P.smem = (words + (P.xs ? P.len : 0)) * 8;
+    // a cluster's kernel has x in shared memory always
+    if (P.nc <= max_nc && P.smem <= kSmemMax && (team == 2 || P.xs)) P.team = team;
+  };
+  if (n <= kClusterCells && max_cluster > 0) {
+    int blocks = 1;
+    while (blocks < max_cluster && (int64_t)blocks * kClusterThreads < n) blocks *= 2;
+    fill(1, blocks, kClusterNC, true);
+  }
+  if (!P.team) fill(2, num_sms, kGridNC, true);
+  if (!P.team) fill(2, num_sms, kGridNC, false);
+  return P;
+}
+
+// Largest cluster size (16, 8, ... 1; 0 on failure) `fn` can run at with the
+// most shared memory, and its opt-ins, once per kernel and device.
+inline int cluster_limit(const void* fn, int threads) {
+  static std::mutex mu;
+  static std::map<std::pair<const void*, int>, int> cache;
+  std::lock_guard<std::mutex> lock(mu);
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  auto it = cache.find({fn, dev});
+  if (it != cache.end()) return it->second;
+  int best = 0;
+  if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMax) == cudaSuccess &&
+      cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess) {
+    for (int c = kMaxCluster; c >= 1 && !best; c /= 2) {
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = c;
+      cfg.blockDim = threads;
+      cfg.dynamicSmemBytes = kSmemMax;
+      cudaLaunchAttribute at[1];
+      at[0].id = cudaLaunchAttributeClusterDimension;
+      at[0].val.clusterDim.x = c;
+      at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+      cfg.attrs = at;
+      cfg.numAttrs = 1;
+      int num = 0;
+      if (cudaOccupancyMaxActiveClusters(&num, fn, &cfg) == cudaSuccess && num >= 1) best = c;
+      else cudaGetLastError();
+    }
+  }
+  cudaGetLastError();
+  return cache[{fn, dev}] = best;
+}
+
+template <typename... KArgs, typename... Args>
+cudaError_t launch_cluster(void (*kernel)(KArgs...), int blocks, int cluster, int threads,
+                           size_t smem, cudaStream_t st, Args&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = blocks;
+  cfg.blockDim = threads;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = cluster;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
+}
+
+struct GridWords {
+  double* partials;
+  unsigned* count;
+  unsigned* error;
+};
+
+template <int THREADS>
+__device__ __forceinline__ ClusterTeam<THREADS> cluster_team(TeamSmem* ts, uint32_t len, FastDiv dlen) {
+  ClusterTeam<THREADS> T;
+  uint32_t r, s;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(s));
+  T.rank_ = (int)r;
+  T.size_ = (int)s;
+  T.len = len;
+  T.dlen = dlen;
+  T.ts = ts;
+  return T;
+}
+
+template <int THREADS>
+__device__ __forceinline__ GridTeam<THREADS> grid_team(TeamSmem* ts, const GridWords& w) {
+  GridTeam<THREADS> T;
+  T.partials = w.partials;
+  T.count = w.count;
+  T.error = w.error;
+  T.timeout_ns = kTimeoutNs;
+  T.rank_ = blockIdx.x;
+  T.size_ = gridDim.x;
+  T.ts = ts;
+  return T;
+}
+
+// Runs f(std::integral_constant NC) for the smallest instantiated NC >= nc.
+template <int... NCS, class F>
+cudaError_t with_nc(int nc, std::integer_sequence<int, NCS...>, F f) {
+  cudaError_t e = cudaErrorInvalidValue;
+  bool done = false;
+  ((!done && nc <= NCS ? (done = true, e = f(std::integral_constant<int, NCS>{})) : e), ...);
+  return e;
+}
+
+// Zeroes the barrier words and the outcome scalars.
+inline cfdb_status prepare_words(cfdb_context* ctx, const Plan& P, GridWords* w) {
+  if (P.team == 2) {
+    cfdb_status st = ensure_partials(ctx, (size_t)2 * P.blocks * kMaxVals);
+    if (st != CFDB_OK) return st;
+  }
+  w->partials = ctx->partials;
+  w->count = ctx->sync_words;
+  w->error = ctx->sync_words + 2;
+  CFDB_CUDA(ctx, cudaMemsetAsync(ctx->sync_words, 0, 4 * sizeof(unsigned), ctx->stream));
+  CFDB_CUDA(ctx, cudaMemsetAsync(ctx->scalars, 0, 8 * sizeof(double), ctx->stream));
+  return CFDB_OK;
+}
+
+}  // namespace res
+}  // namespace cfdb

@@ -1,0 +1,72 @@
+"""The on-chip Krylov solves (resident.cuh) against the CPU oracle at the edges
+of their dispatch: one block, whole and partial blocks of a cluster, the
+cluster's largest system and the first of the grid team's, both thread counts
+of the grid team, and planes too large to be kept in shared memory.
+
+Both sides run the same method with the same arithmetic up to the order of the
+sums, so after a fixed number of iterations the iterates agree to rounding
+(1e-10 relative L2, the bound of the FP64 parity tests being 1e-9).
+"""
+import numpy as np
+import pytest
+
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+GRIDS = [(2, 2), (23, 22), (32, 16), (31, 33), (129, 63), (192, 192), (193, 192), (700, 433),
+         (703, 433), (7, 5, 3), (33, 33, 33), (200, 190, 3), (61, 43, 40)]
+
+
+def _system(n, seed, outlet):
+    """A SIMPLE-like p' system with variable face coefficients."""
+    dim = len(n)
+    pbc = [("fixed_gradient", 0.0)] * (2 * dim)
+    vbc = [("wall", (0, 0, 0))] * (2 * dim)
+    if outlet:
+        pbc[1] = ("fixed_value", 0.0)
+        vbc[0], vbc[1] = ("inlet", (1.0, 0, 0)), ("outlet", (0, 0, 0))
+    case = O.Case(dim, n, tuple(float(m) for m in n), vbc, pbc)
+    rng = np.random.default_rng(seed)
+    d = [rng.uniform(0.5, 2.0, case.cells()) for _ in range(3)]
+    flux = rng.normal(size=case.faces())
+    return (case,) + O.assemble_pprime(case, 1.0, flux, *d)
+
+
+def _rel(a, b):
+    return float(np.linalg.norm(a - b) / max(np.linalg.norm(b), 1e-300))
+
+
+@pytest.mark.parametrize("n", GRIDS)
+def test_pcg_iterates_match_oracle(ctx, n):
+    from cfdapp_b200.cfdb import LinearSolverSettings, POperator
+    for outlet in (False, True):
+        case, fc, diag, off, rhs = _system(n, 5, outlet)
+        x0 = np.random.default_rng(6).normal(size=case.cells())
+        its = min(40, case.cells() // 4)
+        ref = O.stencil_solve(case, diag, off, rhs, x0=x0, rel_tol=1e-30, max_iterations=its)
+        op = POperator(ctx, len(n), n, tuple(float(m) for m in n), face_coeff=fc,
+                       pinned=not outlet)
+        got = op.solve(rhs, LinearSolverSettings(absolute_tolerance=0.0, relative_tolerance=1e-30,
+                                                 max_iterations=its), x0=x0)
+        assert got.status == ref.status and got.iterations == ref.iterations
+        np.testing.assert_allclose(got.residual_history, ref.history, rtol=1e-8)
+        assert _rel(got.solution, ref.solution) <= 1e-10
+
+
+@pytest.mark.parametrize("n", [(40, 33), (193, 192), (17, 19, 23), (64, 50, 40)])
+def test_pcg_of_the_uniform_operator_matches_its_face_form(ctx, n):
+    """Per-axis tables against the same coefficients as face arrays."""
+    from cfdapp_b200.cfdb import LinearSolverSettings, POperator
+    dim = len(n)
+    length = tuple(float(m) for m in n)
+    case = O.Case(dim, n, length, [("wall", (0, 0, 0))] * (2 * dim),
+                  [("fixed_gradient", 0.0)] * (2 * dim))
+    ones = np.ones(case.cells())
+    fc, _, _, _ = O.assemble_pprime(case, 1.0, np.zeros(case.faces()), ones, ones, ones)
+    b = np.random.default_rng(2).normal(size=case.cells())
+    s = LinearSolverSettings(absolute_tolerance=0.0, relative_tolerance=1e-30, max_iterations=50)
+    tab = POperator(ctx, dim, n, length).solve(b, s)
+    arr = POperator(ctx, dim, n, length, face_coeff=fc).solve(b, s)
+    np.testing.assert_allclose(tab.residual_history, arr.residual_history, rtol=1e-12)
+    assert _rel(tab.solution, arr.solution) <= 1e-13
