@@ -393,6 +393,7 @@ struct Io {
   const double* b;
   double* x;
   double* pub;   // GridTeam: published values (cells), else null
+  double* pub2;  // GridTeam, BiCGSTAB: published s (cells)
   double* inv;   // scratch (cells) for M^-1 of a table operator, or null
   double abs_tol, rel_tol;
   int64_t max_it;
@@ -655,6 +656,291 @@ __device__ __forceinline__ void cg_run(const Op& A, uint32_t n, uint32_t len, co
     rz = ab[1];
   }
   finish(CFDB_SOLVER_MAX_ITERATIONS, P.max_it, res_cur);
+}
+
+// (A v^)(c), v^ = v (or, PREC, M^-1 v), v in this block's shared array and,
+// past the range's ends, published by the team; the z-neighbours come with
+// the call (see gather_z).
+template <bool PREC, class Op, class Team>
+__device__ __forceinline__ double neighbour(const Op& A, const Team& T, double coupling,
+                                            const Range& R, uint32_t lc, int off,
+                                            const double* vec, const double* pub) {
+  if (coupling == 0.0) return 0.0;
+  const uint32_t li = lc + (uint32_t)off, c = R.c0 + lc + (uint32_t)off;
+  const double v = li < R.count ? vec[li] : T.remote(vec, pub, c);
+  return PREC ? v * __ldg(A.pinv + c) : v;
+}
+
+// out = A v^ for the thread's cells.  The z-neighbours of two cells
+// are read before the first is used: in 3D they are all outside the block's
+// range, one trip through the team each.  NC > 0: at most NC cells a thread,
+// their coefficients in registers; NC = 0: any number.
+template <int T, int NC, bool PREC, class Op, class Team>
+__device__ __forceinline__ void spmv(const Op& A, const Cells<Op, NC ? NC : 1, (NC > 0)>& cells,
+                                     const Range& R, const Team& team, const double* vec,
+                                     const double* pub, double* out) {
+  constexpr int G = NC ? NC : 2;
+  const int sy = A.nx, sz = (int)A.sz;
+  for (uint32_t g = threadIdx.x; g < R.count; g += G * T) {
+    Cf f[G];
+    double lo[G], hi[G];
+#pragma unroll
+    for (int u = 0; u < G; ++u) {
+      const uint32_t lc = g + u * T;
+      if (lc < R.count) {
+        f[u] = cells.at(A, NC ? u : 0, R.c0 + lc);
+        lo[u] = neighbour<PREC>(A, team, f[u].zl, R, lc, -sz, vec, pub);
+        hi[u] = neighbour<PREC>(A, team, f[u].zh, R, lc, sz, vec, pub);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < G; ++u) {
+      const uint32_t lc = g + u * T;
+      if (lc < R.count)
+        out[lc] = A.mul(
+            f[u], PREC ? vec[lc] * f[u].inv : vec[lc],
+            neighbour<PREC>(A, team, f[u].xl, R, lc, -1, vec, pub),
+            neighbour<PREC>(A, team, f[u].xh, R, lc, 1, vec, pub),
+            Op::kDim == 3 ? neighbour<PREC>(A, team, f[u].yl, R, lc, -sy, vec, pub) : 0.0,
+            Op::kDim == 3 ? neighbour<PREC>(A, team, f[u].yh, R, lc, sy, vec, pub) : 0.0, lo[u], hi[u]);
+    }
+  }
+}
+
+// BiCGSTAB with the reference's breakdown and restart tests
+// (BiCGSTAB.cpp:48-275), the arithmetic of krylov_run (stencil_krylov.cuh).
+// The ranges' ends exchange p once (a barrier of its own) and s (with the
+// reduction of |s|^2): five barriers an iteration, four of them reductions.
+// Shared memory (doubles): p, r/s, rHat, v, t and (XS) x, len each.  The
+// loops over a thread's cells stay rolled unless there are at most two: fully
+// unrolled, the addresses of every cell are kept across the iteration and
+// spill.
+template <int T, int NC, bool XS, bool PREC, class Op, class Team>
+__device__ __forceinline__ void bicgstab_run(const Op& A, uint32_t n, uint32_t len, const Io& P,
+                                             Team& team, double* sm) {
+  const Range R = range_of(n, len, team.rank());
+  double* p = sm;
+  double* r = sm + len;  // r, and s between the half steps
+  double* rh = sm + 2 * (size_t)len;
+  double* v = sm + 3 * (size_t)len;
+  double* t = sm + 4 * (size_t)len;
+  double* xs = sm + 5 * (size_t)len;
+  const uint32_t H = A.sz;
+  const bool leader = team.rank() == 0 && threadIdx.x == 0;
+  Cells<Op, NC ? NC : 1, (NC > 0)> cells;
+  cells.template init<T>(A, R);
+  auto each = [&](auto f) {
+    if constexpr (NC > 0) {
+#pragma unroll
+      for (int q = 0; q < NC; ++q) {
+        const uint32_t lc = threadIdx.x + q * T;
+        if (lc < R.count) f(q, lc, R.c0 + lc);
+      }
+    } else {
+#pragma unroll 2
+      for (uint32_t lc = threadIdx.x; lc < R.count; lc += T) f(0, lc, R.c0 + lc);
+    }
+  };
+  auto publish = [&](double* pub, uint32_t lc, double val) {
+    if (Team::kGlobal && (lc < H || lc + H >= R.count)) pub[R.c0 + lc] = val;
+  };
+  auto x_at = [&](uint32_t lc) { return XS ? xs[lc] : P.x[R.c0 + lc]; };
+  auto set_x = [&](uint32_t lc, double val) {
+    if (XS) xs[lc] = val;
+    else P.x[R.c0 + lc] = val;
+  };
+  auto flush_x = [&]() {
+    if (XS) each([&](int, uint32_t lc, uint32_t c) { P.x[c] = xs[lc]; });
+  };
+  auto finish = [&](int status, int64_t it, double fin) {
+    if (leader) {
+      P.out[0] = status;
+      P.out[1] = (double)it;
+      P.out[3] = fin;
+    }
+    flush_x();
+  };
+  const double eps = DBL_EPSILON;
+  auto cancelled = [&](double ip, double nx_, double ny_, double terms) {
+    if (fabs(ip) > eps * nx_ * ny_) return false;
+    return fabs(ip) <= eps * terms;
+  };
+  // r = rHat = b - A x (x in global memory), v = p = 0; (r, r)
+  auto start = [&](double (&o)[1]) -> bool {
+    o[0] = 0.0;
+    each([&](int q, uint32_t lc, uint32_t c) {
+      const Cf f = cells.at(A, q, c);
+      const double rn = __ldg(P.b + c) - apply_global(A, f, c, P.x);
+      r[lc] = rn;
+      rh[lc] = rn;
+      v[lc] = 0.0;
+      p[lc] = 0.0;
+      o[0] += rn * rn;
+    });
+    return team.reduce(o);
+  };
+  if (XS) each([&](int, uint32_t lc, uint32_t c) { xs[lc] = __ldcg(P.x + c); });
+  double tot[3], one[1];
+  if (!start(one)) return;
+  const double b0 = sqrt(one[0]);
+  if (leader) {
+    P.out[2] = b0;
+    P.out[4] = 0.0;
+    if (P.hist_cap > 0) P.hist[0] = b0;
+  }
+  auto conv = [&](double res) {
+    return (res <= P.abs_tol) || ((b0 > 0.0) && (res / b0 <= P.rel_tol));
+  };
+  if (b0 == 0.0 || conv(b0)) return finish(CFDB_SOLVER_CONVERGED, 0, b0);
+  double rhoOld = 1.0, alpha = 1.0, omega = 1.0;
+  int64_t completed = 0, restarts = 0, hc = 1;
+  double rHatNorm = b0, rNorm = b0, restartResidual = b0, lastHist = b0;
+  double rho = one[0], rhoTerms = one[0];
+  auto push = [&](double val) {
+    if (leader && hc < P.hist_cap) P.hist[hc] = val;
+    ++hc;
+  };
+  // restart (BiCGSTAB.cpp:127-151): 0 restarted, 1 converged, 2 stop
+  auto restart = [&](int& outcome) -> bool {
+    outcome = 2;
+    if (!(rNorm < restartResidual)) return true;
+    flush_x();
+    if (!team.sync()) return false;
+    double o[1];
+    if (!start(o)) return false;
+    rNorm = sqrt(o[0]);
+    if (!isfinite(rNorm)) return true;
+    if (conv(rNorm)) {
+      outcome = 1;
+      return true;
+    }
+    rHatNorm = rNorm;
+    restartResidual = rNorm;
+    rhoOld = 1.0;
+    alpha = 1.0;
+    omega = 1.0;
+    rho = o[0];
+    rhoTerms = o[0];
+    ++restarts;
+    if (leader) P.out[4] = (double)restarts;
+    outcome = 0;
+    return true;
+  };
+  while (completed < P.max_it) {
+    const int64_t iter = completed + 1;
+    if (!isfinite(rho)) return finish(CFDB_SOLVER_BREAKDOWN, completed, rNorm);
+    int oc = 0;
+    if (cancelled(rho, rHatNorm, rNorm, rhoTerms)) {
+      if (!restart(oc)) return;
+      if (oc == 0) continue;
+      return finish(oc == 1 ? CFDB_SOLVER_CONVERGED : CFDB_SOLVER_BREAKDOWN, completed, rNorm);
+    }
+    const double beta = (rho / rhoOld) * (alpha / omega);
+    if (!isfinite(beta)) return finish(CFDB_SOLVER_BREAKDOWN, completed, rNorm);
+    // p = r + (p - v omega) beta
+    each([&](int, uint32_t lc, uint32_t) {
+      const double val = r[lc] + (p[lc] - v[lc] * omega) * beta;
+      p[lc] = val;
+      publish(P.pub, lc, val);
+    });
+    if (!team.sync()) return;
+    // v = A p^; (rHat, v), |v|^2, sum |rHat_i v_i|
+    tot[0] = tot[1] = tot[2] = 0.0;
+    spmv<T, NC, PREC>(A, cells, R, team, p, P.pub, v);
+    each([&](int, uint32_t lc, uint32_t) {
+      const double rhv = rh[lc] * v[lc];
+      tot[0] += rhv;
+      tot[1] += v[lc] * v[lc];
+      tot[2] += fabs(rhv);
+    });
+    if (!team.reduce(tot)) return;
+    const double rHatDotV = tot[0];
+    if (!isfinite(rHatDotV)) return finish(CFDB_SOLVER_BREAKDOWN, completed, rNorm);
+    if (cancelled(rHatDotV, rHatNorm, sqrt(tot[1]), tot[2])) {
+      if (!restart(oc)) return;
+      if (oc == 0) continue;
+      return finish(oc == 1 ? CFDB_SOLVER_CONVERGED : CFDB_SOLVER_BREAKDOWN, completed, rNorm);
+    }
+    alpha = rho / rHatDotV;
+    if (!isfinite(alpha)) return finish(CFDB_SOLVER_BREAKDOWN, completed, rNorm);
+    // s = r - v alpha; |s|^2
+    one[0] = 0.0;
+    each([&](int, uint32_t lc, uint32_t) {
+      const double sv = r[lc] - v[lc] * alpha;
+      r[lc] = sv;
+      publish(P.pub2, lc, sv);
+      one[0] += sv * sv;
+    });
+    if (!team.reduce(one)) return;
+    const double sNorm = sqrt(one[0]);
+    if (!isfinite(sNorm)) {
+      push(sNorm);
+      return finish(CFDB_SOLVER_NONFINITE_RESIDUAL, iter, sNorm);
+    }
+    if (conv(sNorm)) {
+      each([&](int q, uint32_t lc, uint32_t c) {
+        const double ph = PREC ? p[lc] * cells.inverse(A, q, c) : p[lc];
+        set_x(lc, x_at(lc) + ph * alpha);
+      });
+      push(sNorm);
+      return finish(CFDB_SOLVER_CONVERGED, iter, sNorm);
+    }
+    // t = A s^; t.t, t.s, sum |t_i s_i|
+    tot[0] = tot[1] = tot[2] = 0.0;
+    spmv<T, NC, PREC>(A, cells, R, team, r, P.pub2, t);
+    each([&](int, uint32_t lc, uint32_t) {
+      const double tsv = t[lc] * r[lc];
+      tot[0] += t[lc] * t[lc];
+      tot[1] += tsv;
+      tot[2] += fabs(tsv);
+    });
+    if (!team.reduce(tot)) return;
+    const double tDotT = tot[0], tDotS = tot[1];
+    if (!isfinite(tDotT) || tDotT < DBL_MIN) return finish(CFDB_SOLVER_BREAKDOWN, completed, rNorm);
+    if (!isfinite(tDotS)) return finish(CFDB_SOLVER_BREAKDOWN, completed, rNorm);
+    if (cancelled(tDotS, sqrt(tDotT), sNorm, tot[2])) {
+      if (!restart(oc)) return;
+      if (oc == 0) continue;
+      return finish(oc == 1 ? CFDB_SOLVER_CONVERGED : CFDB_SOLVER_BREAKDOWN, completed, rNorm);
+    }
+    omega = tDotS / tDotT;
+    if (!isfinite(omega)) return finish(CFDB_SOLVER_BREAKDOWN, completed, rNorm);
+    // x += p^ alpha; x += s^ omega; r = s - t omega; |r|^2, (rHat, r), sum |rHat_i r_i|
+    tot[0] = tot[1] = tot[2] = 0.0;
+    each([&](int q, uint32_t lc, uint32_t c) {
+      const double sv = r[lc];
+      double ph = p[lc], sh = sv;
+      if (PREC) {
+        const double ivc = cells.inverse(A, q, c);
+        ph *= ivc;
+        sh *= ivc;
+      }
+      double xv = x_at(lc) + ph * alpha;
+      xv = xv + sh * omega;
+      set_x(lc, xv);
+      const double rn = sv - t[lc] * omega;
+      r[lc] = rn;
+      const double rhr = rh[lc] * rn;
+      tot[0] += rn * rn;
+      tot[1] += rhr;
+      tot[2] += fabs(rhr);
+    });
+    if (!team.reduce(tot)) return;
+    const double res = sqrt(tot[0]);
+    rNorm = res;
+    if (!isfinite(res)) {
+      push(res);
+      return finish(CFDB_SOLVER_NONFINITE_RESIDUAL, iter, res);
+    }
+    completed = iter;
+    push(res);
+    lastHist = res;
+    if (conv(res)) return finish(CFDB_SOLVER_CONVERGED, iter, res);
+    rhoOld = rho;
+    rho = tot[1];
+    rhoTerms = tot[2];
+  }
+  finish(CFDB_SOLVER_MAX_ITERATIONS, completed, lastHist);
 }
 
 }  // namespace res

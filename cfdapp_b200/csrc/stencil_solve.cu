@@ -73,6 +73,51 @@ __global__ void k_matrix_finite(StencilMatrix M, const double* b, const double* 
   }
 }
 
+// The persistent kernel that streams its vectors through memory.
+cfdb_status stream_krylov(cfdb_context* ctx, const StencilMatrix& M, StencilWork& W, const double* b,
+                          double* x, int krylov, int jacobi, double abs_tol, double rel_tol,
+                          int64_t max_it, double* hist_dev, int64_t hist_cap) {
+  SParams P{};
+  P.M = M;
+  P.b = b;
+  P.x = x;
+  P.r = W.r;
+  P.rh = W.rh;
+  P.v = W.v;
+  P.p = W.p;
+  P.s = W.s;
+  P.t = W.t;
+  P.krylov = krylov;
+  P.jacobi = jacobi;
+  P.abs_tol = abs_tol;
+  P.rel_tol = rel_tol;
+  P.max_it = max_it;
+  P.hist = hist_dev;
+  P.hist_cap = hist_dev ? hist_cap : 0;
+  int per_sm = 0;
+  CFDB_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, stencil_krylov, kThreads, 0));
+  int64_t grid = std::min<int64_t>((int64_t)std::max(per_sm, 1) * ctx->num_sms, (M.n + kThreads - 1) / kThreads);
+  grid = std::max<int64_t>(grid, 1);
+  cfdb_status st = ensure_partials(ctx, 6 * (size_t)grid);
+  if (st != CFDB_OK) return st;
+  P.partials = ctx->partials;
+  GridSync sync;
+  sync.count = ctx->sync_words;
+  sync.gen = ctx->sync_words + 1;
+  sync.error = ctx->sync_words + 2;
+  sync.nblocks = (unsigned)grid;
+  sync.timeout_ns = kTimeoutNs;
+  P.out = ctx->scalars;
+  CFDB_CUDA(ctx, cudaMemsetAsync(ctx->sync_words, 0, 4 * sizeof(unsigned), ctx->stream));
+  CFDB_CUDA(ctx, cudaMemsetAsync(ctx->scalars, 0, 8 * sizeof(double), ctx->stream));
+  void* args[] = {&P, &sync};
+  CFDB_CUDA(ctx, cudaEventRecord(ctx->ev_k0, ctx->stream));
+  CFDB_CUDA(ctx, cudaLaunchCooperativeKernel((const void*)stencil_krylov, dim3((unsigned)grid),
+                                             dim3(kThreads), args, 0, ctx->stream));
+  CFDB_CUDA(ctx, cudaEventRecord(ctx->ev_k1, ctx->stream));
+  return CFDB_OK;
+}
+
 }  // namespace
 
 cfdb_status stencil_solve(cfdb_context* ctx, const StencilMatrix& Min, StencilWork& W,
@@ -110,44 +155,14 @@ cfdb_status stencil_solve(cfdb_context* ctx, const StencilMatrix& Min, StencilWo
     return CFDB_OK;
   }
   M.inv = jacobi ? W.inv : nullptr;
-  SParams P{};
-  P.M = M;
-  P.b = b;
-  P.x = x;
-  P.r = W.r;
-  P.rh = W.rh;
-  P.v = W.v;
-  P.p = W.p;
-  P.s = W.s;
-  P.t = W.t;
-  P.krylov = krylov;
-  P.jacobi = jacobi;
-  P.abs_tol = abs_tol;
-  P.rel_tol = rel_tol;
-  P.max_it = max_it;
-  P.hist = hist_dev;
-  P.hist_cap = hist_dev ? hist_cap : 0;
-  int per_sm = 0;
-  CFDB_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, stencil_krylov, kThreads, 0));
-  int64_t grid = std::min<int64_t>((int64_t)std::max(per_sm, 1) * ctx->num_sms, (n + kThreads - 1) / kThreads);
-  grid = std::max<int64_t>(grid, 1);
-  cfdb_status st = ensure_partials(ctx, 6 * (size_t)grid);
+  bool on_chip = false;
+  cfdb_status st = resident_stencil_solve(ctx, M, W, b, x, krylov, abs_tol, rel_tol, max_it, hist_dev,
+                                          hist_dev ? hist_cap : 0, &on_chip);
   if (st != CFDB_OK) return st;
-  P.partials = ctx->partials;
-  GridSync sync;
-  sync.count = ctx->sync_words;
-  sync.gen = ctx->sync_words + 1;
-  sync.error = ctx->sync_words + 2;
-  sync.nblocks = (unsigned)grid;
-  sync.timeout_ns = kTimeoutNs;
-  P.out = ctx->scalars;
-  CFDB_CUDA(ctx, cudaMemsetAsync(ctx->sync_words, 0, 4 * sizeof(unsigned), ctx->stream));
-  CFDB_CUDA(ctx, cudaMemsetAsync(ctx->scalars, 0, 8 * sizeof(double), ctx->stream));
-  void* args[] = {&P, &sync};
-  CFDB_CUDA(ctx, cudaEventRecord(ctx->ev_k0, ctx->stream));
-  CFDB_CUDA(ctx, cudaLaunchCooperativeKernel((const void*)stencil_krylov, dim3((unsigned)grid),
-                                             dim3(kThreads), args, 0, ctx->stream));
-  CFDB_CUDA(ctx, cudaEventRecord(ctx->ev_k1, ctx->stream));
+  if (!on_chip) {
+    st = stream_krylov(ctx, M, W, b, x, krylov, jacobi, abs_tol, rel_tol, max_it, hist_dev, hist_cap);
+    if (st != CFDB_OK) return st;
+  }
   count_launch(ctx);
   CFDB_CUDA(ctx, cudaMemcpyAsync(ctx->scalars_host, ctx->scalars, 8 * sizeof(double),
                                  cudaMemcpyDeviceToHost, ctx->stream));

@@ -32,4 +32,12 @@ cfdb_status stencil_solve(cfdb_context* ctx, const StencilMatrix& M, StencilWork
                           double rel_tol, int64_t max_it, double* hist_dev, int64_t hist_cap,
                           cfdb_linear_result* res);
 
+// The same solve with its vectors on chip (resident_bands.cu), launched on
+// the context's stream; *taken: false when the system does not fit.  The
+// outcome lands in the context's scalars as stencil_solve's own kernel's does.
+cfdb_status resident_stencil_solve(cfdb_context* ctx, const StencilMatrix& M, StencilWork& W,
+                                   const double* b, double* x, int krylov, double abs_tol,
+                                   double rel_tol, int64_t max_it, double* hist, int64_t hist_cap,
+                                   bool* taken);
+
 }  // namespace cfdb

@@ -70,3 +70,62 @@ def test_pcg_of_the_uniform_operator_matches_its_face_form(ctx, n):
     arr = POperator(ctx, dim, n, length, face_coeff=fc).solve(b, s)
     np.testing.assert_allclose(tab.residual_history, arr.residual_history, rtol=1e-12)
     assert _rel(tab.solution, arr.solution) <= 1e-13
+
+
+def _csr(diag, off, n):
+    """The rows of a banded system in the reference's column order (host CSR arrays)."""
+    dim = len(n)
+    stride = [1, n[0], n[0] * n[1]]
+    idx = np.arange(int(np.prod(n)))
+    pos = [(idx // stride[a]) % n[a] for a in range(dim)]
+    cols, vals, keep = [], [], []
+    order = [(a, 0) for a in reversed(range(dim))] + [None] + [(a, 1) for a in range(dim)]
+    for o in order:
+        if o is None:
+            c, v, k = idx, diag, np.ones(len(idx), bool)
+        else:
+            a, s = o
+            c, v = idx + (stride[a] if s else -stride[a]), off[2 * a + s]
+            k = pos[a] < n[a] - 1 if s else pos[a] > 0
+        cols.append(c)
+        vals.append(v)
+        keep.append(k)
+    cols, vals, keep = (np.stack(q, axis=1) for q in (cols, vals, keep))
+    ro = np.concatenate([[0], np.cumsum(keep.sum(axis=1))])
+    return ro, cols[keep], vals[keep]
+
+
+@pytest.mark.parametrize("n", GRIDS)
+@pytest.mark.parametrize("method", ["bicgstab", "cg"])
+@pytest.mark.parametrize("jacobi", [False, True])
+def test_band_solves_match_oracle(ctx, n, method, jacobi):
+    """A diagonally dominant banded system (symmetric for CG, upwind-like for BiCGSTAB)
+    through the CSR entry point."""
+    from cfdapp_b200.cfdb import CsrSolver, LinearSolverSettings
+    dim = len(n)
+    case = O.Case(dim, n, tuple(float(m) for m in n), [("wall", (0, 0, 0))] * (2 * dim),
+                  [("fixed_gradient", 0.0)] * (2 * dim))
+    cells = case.cells()
+    rng = np.random.default_rng(8)
+    stride = [1, n[0], n[0] * n[1]]
+    idx = np.arange(cells)
+    off = [np.zeros(cells) for _ in range(6)]
+    total = np.zeros(cells)
+    for a in range(dim):
+        inner = (idx // stride[a]) % n[a] < n[a] - 1
+        lo_of = idx[inner]
+        w = -rng.uniform(0.5, 1.5, len(lo_of))
+        off[2 * a + 1][lo_of] = w
+        off[2 * a][lo_of + stride[a]] = w if method == "cg" else w * rng.uniform(0.2, 1.0, len(w))
+        total += np.abs(off[2 * a]) + np.abs(off[2 * a + 1])
+    diag = (total + 0.05) / 0.8
+    b, x0 = rng.normal(size=cells), rng.normal(size=cells)
+    its = min(6, cells // 2)
+    ref = O.stencil_solve(case, diag, off, b, x0=x0, solver=method, jacobi=jacobi, rel_tol=1e-30,
+                          max_iterations=its)
+    s = LinearSolverSettings(type=method, preconditioner="jacobi" if jacobi else "none",
+                             absolute_tolerance=0.0, relative_tolerance=1e-30, max_iterations=its)
+    got = CsrSolver(ctx).solve(*_csr(diag, off, n), b, s, x0=x0)
+    assert got.status == ref.status and got.iterations == ref.iterations
+    np.testing.assert_allclose(got.residual_history, ref.history, rtol=1e-8)
+    assert _rel(got.solution, ref.solution) <= 1e-10
