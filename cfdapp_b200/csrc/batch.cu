@@ -31,6 +31,7 @@
 #include "cfdb.h"
 #include "cfdb_internal.cuh"
 #include "grid_sync.cuh"
+#include "resident_launch.cuh"
 #include "simple_kernels.cuh"
 #include "stencil_krylov.cuh"
 
@@ -76,7 +77,94 @@ struct KArgs {
   double* kpart;    // 6 doubles per block
   double* kout;     // kKoutStride doubles per (mode, case)
   int record;       // 1: update the case records (0 while tuning)
+  const int* order;  // k_batch_cluster: the case of every cluster, heaviest first
 };
+
+__device__ __forceinline__ double* case_out(const KArgs& A, int k) {
+  return A.kout + (size_t)(A.mode * A.B.ncases + k) * kKoutStride;
+}
+
+// Whether case k takes part in this solve stage; a case whose fields went
+// non-finite earlier in the iteration stops at the p' stage.
+__device__ __forceinline__ bool case_runs(const KArgs& A, int k, bool leader) {
+  const BatchDev& B = A.B;
+  if (!B.active[k]) return false;
+  if (A.mode == 1 && B.flags[(size_t)BF_NONFINITE * B.ncases + k] != 0u) {
+    if (leader && A.record) {
+      B.status[k] = CFDB_SIMPLE_NONFINITE_STATE;
+      B.active[k] = 0;
+    }
+    return false;
+  }
+  return true;
+}
+
+// The input checks the stages before left as flags; the outcome of a system
+// that fails them.
+__device__ __forceinline__ bool case_input_ok(const KArgs& A, int k, bool leader) {
+  const unsigned fl = A.B.flags[(size_t)(A.mode == 0 ? BF_MOM0 + A.comp : BF_PP) * A.B.ncases + k];
+  const bool bad_input = (fl & BFLAG_NONFINITE_INPUT) != 0u;
+  const bool bad_system = A.jacobi && (fl & BFLAG_INVALID_SYSTEM);
+  if (leader && (bad_input || bad_system))
+    case_out(A, k)[krylov::O_STATUS] = bad_input ? CFDB_SOLVER_NONFINITE_INPUT : CFDB_SOLVER_INVALID_SYSTEM;
+  return !bad_input && !bad_system;
+}
+
+// Case k's system in the pools.
+__device__ __forceinline__ krylov::SParams case_system(const KArgs& A, int k) {
+  const BatchDev& B = A.B;
+  const BCase& K = B.cases[k];
+  const int64_t o = K.c0;
+  krylov::SParams P{};
+  P.M.dim = K.G.dim;
+  P.M.nx = K.G.n[0];
+  P.M.ny = K.G.n[1];
+  P.M.nz = K.G.n[2];
+  P.M.n = K.G.nc;
+  P.M.sy = K.G.stride[1];
+  P.M.sz = K.G.stride[2];
+  P.M.diag = (A.mode == 0 ? B.mdiag[A.comp] : B.pdiag) + o;
+  for (int q = 0; q < 6; ++q) P.M.off[q] = (A.mode == 0 ? B.moff[q] : B.poff[q]) + o;
+  P.M.inv = A.jacobi ? B.kinv + o : nullptr;
+  P.b = (A.mode == 0 ? B.mrhs : B.prhs) + o;
+  P.x = (A.mode == 0 ? B.Us[A.comp] : B.pp) + o;
+  P.r = B.kr + o;
+  P.rh = B.krh + o;
+  P.v = B.kv + o;
+  P.p = B.kp + o;
+  P.s = B.ks + o;
+  P.t = B.kt + o;
+  P.krylov = A.krylov;
+  P.jacobi = A.jacobi;
+  P.abs_tol = A.abs_tol;
+  P.rel_tol = A.rel_tol;
+  P.max_it = A.max_it;
+  P.hist = nullptr;
+  P.hist_cap = 0;
+  P.out = case_out(A, k);
+  return P;
+}
+
+// The single-case session's outcome rules, by one thread after the solve.
+__device__ __forceinline__ void case_record(const KArgs& A, int k) {
+  if (!A.record) return;
+  const BatchDev& B = A.B;
+  const double* out = case_out(A, k);
+  const int st = (int)out[krylov::O_STATUS];
+  double* R = B.res + (size_t)k * BR_COUNT;
+  if (st != CFDB_SOLVER_CONVERGED) {
+    B.status[k] = A.mode == 0 ? CFDB_SIMPLE_MOMENTUM_FAILURE : CFDB_SIMPLE_PRESSURE_FAILURE;
+    B.active[k] = 0;
+    return;
+  }
+  if (A.mode == 0) {
+    R[BR_IU + A.comp] = out[krylov::O_B0];
+    B.mom_it[k] += (int64_t)out[krylov::O_ITER];
+  } else {
+    R[BR_IP] = out[krylov::O_B0];
+    B.p_it[k] += (int64_t)out[krylov::O_ITER];
+  }
+}
 
 // Every case's linear solve of one stage; the leader of each team then
 // applies the single-case session's outcome rules (simple.cu
@@ -87,7 +175,8 @@ struct KArgs {
 // Five resident blocks per SM (48 registers, some spilled to L1): the team
 // solves are latency-bound; measured on the 64-case batch, an outer iteration
 // takes 297 ms with two blocks per SM, 222 ms with three, 197 ms with four
-// and 187 ms with five.
+// and 187 ms with five.  (The body spells out what the helpers above do for
+// the cluster kernel: built on them it spills more, 211 against 185 ms.)
 __global__ void __launch_bounds__(krylov::kThreads, 5) k_batch_krylov(KArgs A) {
   const int k = A.block_case[blockIdx.x];
   if (k < 0) return;
@@ -189,6 +278,46 @@ __global__ void __launch_bounds__(krylov::kThreads, 5) k_batch_krylov(KArgs A) {
   }
 }
 
+// The same stage for the cases whose vectors fit the shared memory of one
+// cluster: a cluster of 16 blocks per case, on chip (resident.cuh).  Seven
+// clusters run at once (112 SMs); the others start as these finish, heaviest
+// case first.  An outer iteration of 12 cavities and channels of 48^2 to
+// 256^2 with FP64 CG takes 26.6 ms, against 51.6 ms with teams.
+template <int DIM, int NC, int KRYLOV, bool PREC>
+__global__ void __launch_bounds__(res::kClusterThreads, 1) k_batch_cluster(KArgs A) {
+  extern __shared__ __align__(16) double sm[];
+  __shared__ res::TeamSmem ts;
+  const int k = A.order[blockIdx.x / res::kMaxCluster];
+  const bool leader = blockIdx.x % res::kMaxCluster == 0 && threadIdx.x == 0;
+  if (!case_runs(A, k, leader)) return;
+  if (case_input_ok(A, k, leader)) {
+    const krylov::SParams S = case_system(A, k);
+    if (leader) S.out[krylov::O_STATUS] = -1.0;
+    const uint32_t n = (uint32_t)S.M.n, len = (n + res::kMaxCluster - 1) / res::kMaxCluster;
+    auto team = res::cluster_team<res::kClusterThreads>(&ts, len, res::fast_div(len));
+    const res::BandOp<DIM> Op = res::band_op<DIM>(S.M);
+    res::Io P{};
+    P.b = S.b;
+    P.x = S.x;
+    P.abs_tol = S.abs_tol;
+    P.rel_tol = S.rel_tol;
+    P.max_it = S.max_it;
+    P.out = S.out;
+    if constexpr (KRYLOV == 1) res::bicgstab_run<res::kClusterThreads, 0, true, PREC>(Op, n, len, P, team, sm);
+    else res::cg_run<res::kClusterThreads, NC, false, true, true>(Op, n, len, P, team, sm);
+  }
+  if (leader) case_record(A, k);
+}
+
+using BatchKernel = void (*)(KArgs);
+// The instance for a dimension, method and most cells per thread.
+template <int DIM>
+BatchKernel cluster_kernel_of(int krylov, bool prec, int nc) {
+  if (krylov == 1) return prec ? k_batch_cluster<DIM, 1, 1, true> : k_batch_cluster<DIM, 1, 1, false>;
+  return nc <= 2 ? k_batch_cluster<DIM, 2, 0, false>
+                 : (nc <= 4 ? k_batch_cluster<DIM, 4, 0, false> : k_batch_cluster<DIM, 8, 0, false>);
+}
+
 // The learned p' solves' outcomes (lout: status, iterations, initial
 // residual per case, written by the host) applied with k_batch_krylov's
 // record rules: a case whose fields went non-finite stops with
@@ -246,6 +375,14 @@ struct cfdb_batch {
   int *d_bcase_m = nullptr, *d_tfirst_m = nullptr, *d_bcase_p = nullptr, *d_tfirst_p = nullptr;
   unsigned *d_bar = nullptr, *d_err = nullptr;
   double *d_kpart = nullptr, *d_kout = nullptr;
+  // solves by one cluster per case, per mode (0 momentum, 1 p'): the kernel,
+  // its shared memory, and the cases' order (device)
+  struct Clusters {
+    bool on = false;
+    BatchKernel kernel = nullptr;
+    size_t smem = 0;
+    int* d_order = nullptr;
+  } clusters[2];
   std::vector<int> h_active;  // host view of the active set the teams were planned for
   std::vector<double> h_pweight;
   // tuning and launch shapes
@@ -380,9 +517,40 @@ void launch_krylov(cfdb_batch* b, int mode, int comp, int record, cudaStream_t s
   A.kpart = b->d_kpart;
   A.kout = b->d_kout;
   A.record = record;
-  k_batch_krylov<<<b->kgrid, krylov::kThreads, 0, s>>>(A);
+  const cfdb_batch::Clusters& C = b->clusters[mode];
+  if (C.on) {
+    A.order = C.d_order;
+    res::launch_cluster(C.kernel, b->n * res::kMaxCluster, res::kMaxCluster, res::kClusterThreads,
+                        C.smem, s, A);
+  } else {
+    k_batch_krylov<<<b->kgrid, krylov::kThreads, 0, s>>>(A);
+  }
   b->launches_per_iteration += 1;
   mark(b, mode == 0 ? -1 : -2, s);
+}
+
+// Whether a mode's solves run in clusters, and their kernel: FP64 ones, when
+// every case's vectors fit the shared memory of kMaxCluster blocks (65536
+// cells).  With a larger case in it the whole batch keeps to teams, which
+// share the GPU among all cases at once.
+cfdb_status plan_clusters(cfdb_batch* b, int mode) {
+  const cfdb_linear_settings& L = mode == 0 ? b->st.momentum : b->st.pressure;
+  cfdb_batch::Clusters& C = b->clusters[mode];
+  const bool prec = L.preconditioner == CFDB_PRECOND_JACOBI;
+  if (mode == 1 && L.precision != CFDB_PRECISION_FP64) return CFDB_OK;
+  size_t longest = 0;
+  for (int k = 0; k < b->n; ++k) {
+    const int64_t reach = b->dim == 3 ? b->hc[k].G.stride[2] : b->hc[k].G.stride[1];
+    const size_t need = res::cluster_smem(b->cells[k], reach, L.krylov, res::kClusterNC);
+    if (need == 0) return CFDB_OK;
+    C.smem = std::max(C.smem, need);
+    longest = std::max(longest, (size_t)((b->cells[k] + res::kMaxCluster - 1) / res::kMaxCluster));
+  }
+  const int nc = (int)((longest + res::kClusterThreads - 1) / res::kClusterThreads);
+  C.kernel = b->dim == 2 ? cluster_kernel_of<2>(L.krylov, prec, nc) : cluster_kernel_of<3>(L.krylov, prec, nc);
+  if (res::cluster_limit((const void*)C.kernel, res::kClusterThreads) < res::kMaxCluster) return CFDB_OK;
+  C.on = true;
+  return dalloc(b, &C.d_order, b->n);
 }
 
 // Stages of an outer iteration up to the p' solve (record = 0: the linear
@@ -545,6 +713,12 @@ cfdb_status upload_tiles(cfdb_batch* b) {
 cfdb_status upload_teams(cfdb_batch* b, int mode, const std::vector<double>& w) {
   const int n = b->n;
   std::vector<int> tf(n + 1), bc(b->kgrid);
+  const cfdb_batch::Clusters& C = b->clusters[mode];
+  std::vector<int> order;
+  if (C.on) {
+    for (int k = 0; k < n; ++k) order.push_back(k);
+    std::stable_sort(order.begin(), order.end(), [&](int p, int q) { return w[p] > w[q]; });
+  }
   cfdb_status rc = cfdb_batch_plan_teams(n, w.data(), b->cells.data(), b->h_active.data(), b->kgrid,
                                          kMinCellsPerBlock, tf.data(), bc.data());
   if (rc != CFDB_OK) return set_error(b->ctx, rc, "more active cases than Krylov blocks");
@@ -553,6 +727,9 @@ cfdb_status upload_teams(cfdb_batch* b, int mode, const std::vector<double>& w) 
                                     sizeof(int) * (n + 1), cudaMemcpyHostToDevice, s));
   CFDB_CUDA(b->ctx, cudaMemcpyAsync(mode == 0 ? b->d_bcase_m : b->d_bcase_p, bc.data(),
                                     sizeof(int) * b->kgrid, cudaMemcpyHostToDevice, s));
+  if (!order.empty())
+    CFDB_CUDA(b->ctx, cudaMemcpyAsync(C.d_order, order.data(), sizeof(int) * order.size(),
+                                      cudaMemcpyHostToDevice, s));
   // the host vectors die here: finish the copies
   CFDB_CUDA(b->ctx, cudaStreamSynchronize(s));
   return CFDB_OK;
@@ -867,6 +1044,8 @@ cfdb_status cfdb_batch_create(cfdb_context* ctx, int ncases, const cfdb_simple_c
       (rc = dalloc(b.get(), &b->d_kpart, 6 * (size_t)b->kgrid)) ||
       (rc = dalloc(b.get(), &b->d_kout, 2 * (size_t)ncases * kKoutStride)))
     return rc;
+  for (int mode = 0; mode < 2; ++mode)
+    if ((rc = plan_clusters(b.get(), mode))) return rc;
   CFDB_CUDA(ctx, cudaMallocHost((void**)&b->h_nactive, sizeof(int)));
   CFDB_CUDA(ctx, cudaMallocHost((void**)&b->h_err, sizeof(unsigned)));
   CFDB_CUDA(ctx, cudaMallocHost((void**)&b->h_kout, sizeof(double) * 2 * ncases * kKoutStride));

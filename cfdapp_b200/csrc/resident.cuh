@@ -49,7 +49,7 @@ struct FastDiv {
     return (uint32_t)(((uint64_t)c * m) >> s);
   }
 };
-inline FastDiv fast_div(uint32_t d) {
+__host__ __device__ inline FastDiv fast_div(uint32_t d) {
   FastDiv f;
   uint32_t l = 0;
   while ((1ull << l) < d) ++l;
@@ -185,8 +185,9 @@ struct BandOp {
 };
 
 template <int DIM>
-BandOp<DIM> band_op(const StencilMatrix& M) {
-  BandOp<DIM> A{};
+__host__ __device__ inline BandOp<DIM> band_op(const StencilMatrix& M) {
+  BandOp<DIM> A;
+  A.oyl = A.oyh = nullptr;
   A.diag = M.diag;
   A.oxl = M.off[0];
   A.oxh = M.off[1];

@@ -97,6 +97,15 @@ inline Plan bicgstab_plan(int64_t n, int num_sms, int max_cluster) {
   return P;
 }
 
+// Shared memory of one cluster of kMaxCluster blocks running the CG or the
+// BiCGSTAB of n cells with everything in shared memory; 0: does not fit.
+inline size_t cluster_smem(int64_t n, int64_t reach, int krylov, int max_nc) {
+  const size_t len = (size_t)((n + kMaxCluster - 1) / kMaxCluster);
+  const size_t words = krylov == 1 ? 6 * len : 4 * len + 2 * (size_t)reach;
+  if (words * 8 > kSmemMax || len > (size_t)max_nc * kClusterThreads) return 0;
+  return words * 8;
+}
+
 // Largest cluster size (16, 8, ... 1; 0 on failure) `fn` can run at with the
 // most shared memory, and its opt-ins, once per kernel and device.
 inline int cluster_limit(const void* fn, int threads) {

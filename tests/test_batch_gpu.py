@@ -274,3 +274,33 @@ def test_batch_learned_pprime_matches_reference(ctx, name):
     assert _rel(f, g["flux"]) <= 1e-6
     assert b.results()[0]["status"] == "Converged"
     b.close()
+
+
+@pytest.mark.parametrize("method", ["cg", "bicgstab"])
+def test_batch_clusters_and_teams_agree(ctx, method):
+    """A batch whose cases all fit a cluster solves on chip; with one case that does not, the
+    same cases go through block teams.  Both run the same methods, each to its own order of the
+    sums, so after a few outer iterations (linear solves to 1e-12) the fields agree to 1e-8
+    (what the solves' tolerance leaves after the coupling of a few outer iterations)."""
+    from cfdapp_b200.cfdb import Batch, LinearSolverSettings, SIMPLESettings, SimpleCase
+    ps = LinearSolverSettings(type=method, preconditioner="jacobi", absolute_tolerance=0.0,
+                              relative_tolerance=1e-12, max_iterations=20000)
+    ms = LinearSolverSettings(type="bicgstab", preconditioner="none", absolute_tolerance=0.0,
+                              relative_tolerance=1e-12, max_iterations=2000)
+    st = SIMPLESettings(max_iterations=3, momentum_solver=ms, pressure_solver=ps)
+    small = [SimpleCase.cavity(2, 17), SimpleCase.channel(48, 24, 2.0, 1.0),
+             SimpleCase.cavity(2, 96)]
+    large = SimpleCase.cavity(2, 300)  # 90 000 cells: past a cluster's shared memory
+    got = []
+    for cases in (small, small + [large]):
+        b = Batch(ctx, cases, st)
+        for k in range(len(cases)):
+            b.set_state(k)
+        b.iterate(3)
+        got.append([b.get_state(k) for k in range(len(small))])
+        assert all(r["status"] == "MaxIterations" for r in b.results()[:len(small)])
+        b.close()
+    for one, other in zip(*got):
+        for a, c in zip(one, other):
+            if a.size:
+                assert np.linalg.norm(a - c) <= 1e-8 * np.linalg.norm(c)
