@@ -16,7 +16,8 @@
 // 2x2x2 children of a coarse cell are summed inside one block (shuffle in x,
 // shared memory in y, a register across the z pair) -- deterministic, no
 // atomics.  All levels at or below 4096 cells run inside ONE thread block
-// with their data in shared memory.
+// with their data in shared memory; the levels above them up to 32768 cells,
+// and the whole solve of a small system, on one cluster (mg_cluster.cuh).
 //
 // Reductions are deterministic without a grid barrier: every block stores its
 // partial sums, and the last block to finish (atomic ticket) adds all partials
@@ -37,6 +38,7 @@
 #include "grid_sync.cuh"
 #include "mg.cuh"
 #include "pcg_internal.cuh"
+#include "resident_launch.cuh"
 
 namespace cfdb {
 
@@ -615,7 +617,9 @@ struct CoarseLevel {
   const float* isq;
   float* x_glob;      // global x (written back for the first coarse level)
   const float* r_glob;
-  int off[7];         // shared-memory offsets (floats): fx fy fz isq x r res
+  int off[7];         // shared-memory offsets (floats): fx fy fz isq x r u
+  res::FastDiv dx, dy;
+  int warps;          // warps that work on the level
 };
 
 struct CoarsePlan {
@@ -692,12 +696,11 @@ __device__ __forceinline__ float coarse_conv(const CoarseGeo<DIM>& G, const Kern
 // instruction issue.  Cell coordinates come from a float reciprocal (exact
 // below 2^22 cells); the coarsest level's damped-Jacobi sweeps run on only
 // the warps that own its cells (a named barrier instead of the whole block).
+
+// Zeroes the padded vectors (their halos stay zero).
 template <int DIM>
-__global__ void __launch_bounds__(kCoarseThreads) k_coarse(CoarsePlan P) {
-  extern __shared__ float4 smem4[];
-  float* sm = reinterpret_cast<float*>(smem4);
+__device__ __forceinline__ void coarse_clear(const CoarsePlan& P, float* sm) {
   const int tid = threadIdx.x, nt = blockDim.x;
-  // zero the padded vectors (their halos stay zero)
   for (int l = 0; l < P.count; ++l) {
     const CoarseLevel& c = P.lv[l];
     const int words = (coarse_padded(DIM, c.n) + 3) >> 2;
@@ -708,28 +711,70 @@ __global__ void __launch_bounds__(kCoarseThreads) k_coarse(CoarsePlan P) {
       r4[q] = make_float4(0.f, 0.f, 0.f, 0.f);
     }
   }
-  pdl_enter();
-  // 16-byte copies over the body of each array (every source is its own
-  // allocation, every destination 16-byte aligned), 4-byte ones for the tail
-  auto fetch = [&](float* dst, const float* src, int count) {
-    const int body = count & ~3;
-    for (int q = 4 * tid; q < body; q += 4 * nt) cp16(dst + q, src + q, true);
-    for (int q = body + tid; q < count; q += nt) cp4(dst + q, src + q, true);
-  };
+}
+
+// 16-byte copies over the body of an array (every source is its own
+// allocation, every destination 16-byte aligned), 4-byte ones for the tail
+__device__ __forceinline__ void coarse_fetch(float* dst, const float* src, int count) {
+  const int tid = threadIdx.x, nt = blockDim.x;
+  const int body = count & ~3;
+  for (int q = 4 * tid; q < body; q += 4 * nt) cp16(dst + q, src + q, true);
+  for (int q = body + tid; q < count; q += nt) cp4(dst + q, src + q, true);
+}
+
+// Issues the copies of every level's couplings and scales.
+template <int DIM>
+__device__ __forceinline__ void coarse_fetch_levels(const CoarsePlan& P, float* sm) {
   for (int l = 0; l < P.count; ++l) {
     const CoarseLevel& c = P.lv[l];
-    fetch(sm + c.off[0], c.f[0], (c.n[0] + 1) * c.n[1] * c.n[2]);
-    if (DIM == 3) fetch(sm + c.off[1], c.f[1], c.n[0] * (c.n[1] + 1) * c.n[2]);
-    fetch(sm + c.off[2], c.f[2], c.n[0] * c.n[1] * (c.n[2] + 1));
-    fetch(sm + c.off[3], c.isq, c.cells);
+    coarse_fetch(sm + c.off[0], c.f[0], (c.n[0] + 1) * c.n[1] * c.n[2]);
+    if (DIM == 3) coarse_fetch(sm + c.off[1], c.f[1], c.n[0] * (c.n[1] + 1) * c.n[2]);
+    coarse_fetch(sm + c.off[2], c.f[2], c.n[0] * c.n[1] * (c.n[2] + 1));
+    coarse_fetch(sm + c.off[3], c.isq, c.cells);
   }
-  fetch(sm + P.lv[0].off[5], P.lv[0].r_glob, P.lv[0].cells);
-  cp_commit();
-  cp_wait<0>();
-  __syncthreads();
-  auto level = [&](int l) {
+}
+
+// One cycle over the levels in shared memory: the first level's r is in
+// place; the first level's x (padded) is the result.
+//
+// The cycle is a chain of some 30 short phases, so what counts is the latency
+// of each: a level is worked on by only the warps that own its cells, behind
+// a named barrier of its own (the others wait where they are needed again),
+// the scaled residual u is formed where r is, and prolongation and Jacobi
+// sweeps need no phase of their own (x + c P e is formed as it is read, the
+// sweeps alternate between two vectors).  With it a 24^3 FCG iteration takes
+// 37 us instead of 41, 12^3 21 instead of 26.
+template <int DIM>
+__device__ __forceinline__ void coarse_cycle(const CoarsePlan& P, float* sm) {
+  const int tid = threadIdx.x, warp = tid >> 5;
+  const int last = P.count - 1;
+  // a level as this thread works on it, in registers: its geometry, vectors
+  // and the thread's first cell (on the smaller levels its only one)
+  struct Cell {
+    int i, j, k, c, rest, pc;
+  };
+  struct Level : CoarseGeo<DIM> {
+    int cells, nt, id;
+    res::FastDiv dx, dy;
+    float *x, *r, *u;
+    Cell first;
+    __device__ __forceinline__ Cell cell(int c) const {
+      Cell o;
+      o.c = c;
+      o.rest = (int)dx.div((uint32_t)c);
+      o.i = c - o.rest * this->nx;
+      o.k = DIM == 3 ? (int)dy.div((uint32_t)o.rest) : o.rest;
+      o.j = DIM == 3 ? o.rest - o.k * this->ny : 0;
+      o.pc = this->pad(o.i, o.j, o.k);
+      return o;
+    }
+    __device__ __forceinline__ void sync() const {
+      asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nt) : "memory");
+    }
+  };
+  auto geo = [&](int l) {
     const CoarseLevel& c = P.lv[l];
-    CoarseGeo<DIM> G;
+    Level G;
     G.nx = c.n[0];
     G.ny = c.n[1];
     G.nz = c.n[2];
@@ -739,115 +784,180 @@ __global__ void __launch_bounds__(kCoarseThreads) k_coarse(CoarsePlan P) {
     G.fy = DIM == 3 ? sm + c.off[1] : nullptr;
     G.fz = sm + c.off[2];
     G.isq = sm + c.off[3];
+    G.x = sm + c.off[4];
+    G.r = sm + c.off[5];
+    G.u = sm + c.off[6];
+    G.cells = c.cells;
+    G.nt = 32 * c.warps;
+    G.id = l + 1;
+    G.dx = c.dx;
+    G.dy = c.dy;
+    G.first = G.cell(tid);
     return G;
   };
-  // f(i, j, k, c, rest, pc) for every cell of G, strided over the block
-  auto cells_of = [&](const CoarseGeo<DIM>& G, auto f) {
-    const int cells = G.nx * G.ny * G.nz;
-    const float inx = 1.0f / (float)G.nx, iny = 1.0f / (float)G.ny;
-    for (int c = tid; c < cells; c += nt) {
-      const int rest = __float2int_rz(((float)c + 0.5f) * inx);
-      const int i = c - rest * G.nx;
-      const int k = DIM == 3 ? __float2int_rz(((float)rest + 0.5f) * iny) : rest;
-      const int j = DIM == 3 ? rest - k * G.ny : 0;
-      f(i, j, k, c, rest, G.pad(i, j, k));
-    }
+  // f(cell) for every cell of a level, by its warps
+  auto cells_of = [&](const Level& G, auto f) {
+    if (tid < G.cells) f(G.first);
+    for (int c = tid + G.nt; c < G.cells; c += G.nt) f(G.cell(c));
   };
-  const int last = P.count - 1;
+  auto mine = [&](int l) { return warp < P.lv[l].warps; };
+  // u = D^-1/2 r, or x after the first of the coarsest level's sweeps
+  const int sweeps = P.sweeps, nu = P.nu;
+  auto start = [&](int l, const Level& G, const Cell& q, float r) {
+    const float is = G.isq[q.c];
+    if (l < last) G.u[q.pc] = is * r;
+    else G.x[q.pc] = sweeps > 0 ? 0.8f * (is * is) * r : 0.f;
+  };
+  auto lap = [&](const Level& G, const Cell& q, const float* x) {
+    return coarse_lap<DIM>(G, q.c, q.rest, q.k, q.pc, x);
+  };
+  if (mine(0)) {
+    const Level G = geo(0);
+    cells_of(G, [&](const Cell& q) { start(0, G, q, G.r[q.c]); });
+    G.sync();
+  }
+  int deepest = -1;  // the last level this warp works on
   for (int l = 0; l < last; ++l) {
-    const CoarseGeo<DIM> G = level(l);
-    float* x = sm + P.lv[l].off[4];
-    const float* r = sm + P.lv[l].off[5];
-    float* res = sm + P.lv[l].off[6];
+    if (!mine(l)) break;
+    deepest = l;
+    const Level G = geo(l);
     const Kern& K = P.K[l];
-    cells_of(G, [&](int, int, int, int c, int, int pc) { res[pc] = G.isq[c] * r[c]; });
-    __syncthreads();
-    cells_of(G, [&](int, int, int, int c, int, int pc) { x[pc] = G.isq[c] * coarse_conv<DIM>(G, K, pc, res); });
-    __syncthreads();
-    for (int s = 1; s < P.nu; ++s) {
-      cells_of(G, [&](int, int, int k, int c, int rest, int pc) {
-        res[pc] = G.isq[c] * (r[c] - coarse_lap<DIM>(G, c, rest, k, pc, x));
-      });
-      __syncthreads();
-      cells_of(G, [&](int, int, int, int c, int, int pc) { x[pc] += G.isq[c] * coarse_conv<DIM>(G, K, pc, res); });
-      __syncthreads();
+    cells_of(G, [&](const Cell& q) { G.x[q.pc] = G.isq[q.c] * coarse_conv<DIM>(G, K, q.pc, G.u); });
+    G.sync();
+    for (int s = 1; s < nu; ++s) {
+      cells_of(G, [&](const Cell& q) { G.u[q.pc] = G.isq[q.c] * (G.r[q.c] - lap(G, q, G.x)); });
+      G.sync();
+      cells_of(G, [&](const Cell& q) { G.x[q.pc] += G.isq[q.c] * coarse_conv<DIM>(G, K, q.pc, G.u); });
+      G.sync();
     }
-    cells_of(G, [&](int, int, int k, int c, int rest, int pc) { res[pc] = r[c] - coarse_lap<DIM>(G, c, rest, k, pc, x); });
-    __syncthreads();
+    cells_of(G, [&](const Cell& q) { G.u[q.pc] = G.r[q.c] - lap(G, q, G.x); });
+    G.sync();
+    if (!mine(l + 1)) break;
     // restriction: the sum over the 2 x 2 (x 2) children, (z, y, x) order;
     // children past an odd edge are halo zeros
-    const CoarseGeo<DIM> C = level(l + 1);
-    float* rc = sm + P.lv[l + 1].off[5];
-    cells_of(C, [&](int ci, int cj, int ck, int qc, int, int) {
+    const Level C = geo(l + 1);
+    cells_of(C, [&](const Cell& q) {
       float s = 0.f;
 #pragma unroll
-      for (int u = 0; u < 2; ++u)
+      for (int a = 0; a < 2; ++a)
 #pragma unroll
-        for (int v = 0; v < (DIM == 3 ? 2 : 1); ++v)
+        for (int b = 0; b < (DIM == 3 ? 2 : 1); ++b)
 #pragma unroll
-          for (int t = 0; t < 2; ++t) s += res[G.pad(2 * ci + t, 2 * cj + v, 2 * ck + u)];
-      rc[qc] = s;
+          for (int t = 0; t < 2; ++t) s += G.u[G.pad(2 * q.i + t, 2 * q.j + b, 2 * q.k + a)];
+      C.r[q.c] = s;
+      start(l + 1, C, q, s);
     });
-    __syncthreads();
+    C.sync();
+    deepest = l + 1;
   }
-  {
-    const CoarseGeo<DIM> G = level(last);
-    float* x = sm + P.lv[last].off[4];
-    const float* r = sm + P.lv[last].off[5];
-    float* res = sm + P.lv[last].off[6];
-    const int cells = G.nx * G.ny * G.nz;
-    const int nw = min(32, (cells + 31) / 32);  // warps that own the coarsest cells
-    if (tid < 32 * nw) {
-      auto wsync = [&]() {
-        if (nw == 1) __syncwarp();
-        else asm volatile("bar.sync 1, %0;" ::"r"(32 * nw) : "memory");
-      };
-      const float inx = 1.0f / (float)G.nx, iny = 1.0f / (float)G.ny;
-      for (int s = 0; s < P.sweeps; ++s) {
-        for (int c = tid; c < cells; c += 32 * nw) {
-          const int rest = __float2int_rz(((float)c + 0.5f) * inx);
-          const int i = c - rest * G.nx;
-          const int k = DIM == 3 ? __float2int_rz(((float)rest + 0.5f) * iny) : rest;
-          const int pc = G.pad(i, DIM == 3 ? rest - k * G.ny : 0, k);
-          res[pc] = r[c] - coarse_lap<DIM>(G, c, rest, k, pc, x);
-        }
-        wsync();
-        for (int c = tid; c < cells; c += 32 * nw) {
-          const int rest = __float2int_rz(((float)c + 0.5f) * inx);
-          const int i = c - rest * G.nx;
-          const int k = DIM == 3 ? __float2int_rz(((float)rest + 0.5f) * iny) : rest;
-          const int pc = G.pad(i, DIM == 3 ? rest - k * G.ny : 0, k);
-          const float is = G.isq[c];
-          x[pc] += 0.8f * (is * is) * res[pc];
-        }
-        wsync();
-      }
-    }
-    __syncthreads();
-  }
-  for (int l = last - 1; l >= 0; --l) {
-    const CoarseGeo<DIM> G = level(l);
-    const CoarseGeo<DIM> C = level(l + 1);
-    float* x = sm + P.lv[l].off[4];
-    const float* r = sm + P.lv[l].off[5];
-    float* res = sm + P.lv[l].off[6];
-    const float* ec = sm + P.lv[l + 1].off[4];
-    const float cw = P.cw[l];
-    const Kern& K = P.K[l];
-    cells_of(G, [&](int i, int j, int k, int, int, int pc) { x[pc] += cw * ec[C.pad(i >> 1, j >> 1, k >> 1)]; });
-    __syncthreads();
-    for (int s = 0; s < P.nu; ++s) {
-      cells_of(G, [&](int, int, int k, int c, int rest, int pc) {
-        res[pc] = G.isq[c] * (r[c] - coarse_lap<DIM>(G, c, rest, k, pc, x));
+  if (mine(last)) {
+    deepest = last;
+    const Level G = geo(last);
+    float *x = G.x, *y = G.u;
+    for (int s = 1; s < sweeps; ++s) {
+      cells_of(G, [&](const Cell& q) {
+        const float is = G.isq[q.c];
+        y[q.pc] = x[q.pc] + 0.8f * (is * is) * (G.r[q.c] - lap(G, q, x));
       });
-      __syncthreads();
-      cells_of(G, [&](int, int, int, int c, int, int pc) { x[pc] += G.isq[c] * coarse_conv<DIM>(G, K, pc, res); });
-      __syncthreads();
+      G.sync();
+      float* t = x;
+      x = y;
+      y = t;
+    }
+    if (x != G.x) {  // the result belongs in x
+      cells_of(G, [&](const Cell& q) { y[q.pc] = x[q.pc]; });
+      if (last == 0) G.sync();
     }
   }
-  const CoarseGeo<DIM> G0 = level(0);
-  const float* x0 = sm + P.lv[0].off[4];
-  cells_of(G0, [&](int, int, int, int c, int, int pc) { P.lv[0].x_glob[c] = x0[pc]; });
+  for (int l = min(last - 1, deepest); l >= 0; --l) {
+    const Level G = geo(l);
+    const CoarseLevel& cl = P.lv[l + 1];
+    const int cpx = cl.n[0] + 2, cpz = DIM == 3 ? cpx * (cl.n[1] + 2) : cpx;
+    const float* ec = sm + cl.off[4];
+    const Kern& K = P.K[l];
+    const float cw = P.cw[l];
+    // c P e at a cell, 0 outside the domain (x's own halo is 0)
+    auto e = [&](int i, int j, int k) {
+      const float v = ec[((i >> 1) + 1) + (DIM == 3 ? cpx * ((j >> 1) + 1) : 0) + cpz * ((k >> 1) + 1)];
+      const bool in = i >= 0 && i < G.nx && k >= 0 && k < G.nz && (DIM == 2 || (j >= 0 && j < G.ny));
+      return in ? cw * v : 0.f;
+    };
+    G.sync();  // the level below is done (its warps are among this level's)
+    for (int s = 0; s < nu; ++s) {
+      cells_of(G, [&](const Cell& q) {
+        float ax;
+        if (s == 0) {
+          C7 co;
+          co.xl = G.fx[q.c + q.rest];
+          co.xh = G.fx[q.c + q.rest + 1];
+          co.yl = DIM == 3 ? G.fy[q.c + G.nx * q.k] : 0.f;
+          co.yh = DIM == 3 ? G.fy[q.c + G.nx * q.k + G.nx] : 0.f;
+          co.zl = G.fz[q.c];
+          co.zh = G.fz[q.c + G.nx * G.ny];
+          co.d = ((co.xl + co.xh) + (co.yl + co.yh)) + (co.zl + co.zh);
+          const float* x = G.x + q.pc;
+          ax = apply7(co, x[0] + e(q.i, q.j, q.k), x[-1] + e(q.i - 1, q.j, q.k),
+                      x[1] + e(q.i + 1, q.j, q.k), DIM == 3 ? x[-G.px] + e(q.i, q.j - 1, q.k) : 0.f,
+                      DIM == 3 ? x[G.px] + e(q.i, q.j + 1, q.k) : 0.f, x[-G.pz] + e(q.i, q.j, q.k - 1),
+                      x[G.pz] + e(q.i, q.j, q.k + 1));
+        } else {
+          ax = lap(G, q, G.x);
+        }
+        G.u[q.pc] = G.isq[q.c] * (G.r[q.c] - ax);
+      });
+      G.sync();
+      cells_of(G, [&](const Cell& q) {
+        float v = G.x[q.pc] + G.isq[q.c] * coarse_conv<DIM>(G, K, q.pc, G.u);
+        if (s == 0) v += e(q.i, q.j, q.k);
+        G.x[q.pc] = v;
+      });
+      if (s + 1 < nu) G.sync();
+    }
+  }
+  __syncthreads();
+}
+
+// A plan's copy in shared memory (T: a multiple of 4 bytes), whose levels are
+// indexed at run time: an indexed read of a kernel parameter goes through
+// the constant cache, which these plans (3 KB, read by every warp) thrash.
+template <class T>
+__device__ __forceinline__ const T& to_shared(const T& src, void* dst) {
+  static_assert(sizeof(T) % 4 == 0, "whole words");
+  const unsigned* s = reinterpret_cast<const unsigned*>(&src);
+  unsigned* d = reinterpret_cast<unsigned*>(dst);
+  for (int q = threadIdx.x; q < (int)(sizeof(T) / 4); q += blockDim.x) d[q] = s[q];
+  __syncthreads();
+  return *reinterpret_cast<const T*>(dst);
+}
+// Floats a plan's copy takes at the front of dynamic shared memory.
+template <class T>
+constexpr int plan_words() {
+  return (int)((sizeof(T) + 15) / 16) * 4;
+}
+
+template <int DIM>
+__global__ void __launch_bounds__(kCoarseThreads) k_coarse(const __grid_constant__ CoarsePlan arg) {
+  extern __shared__ float4 smem4[];
+  const CoarsePlan& P = to_shared(arg, smem4);
+  float* sm = reinterpret_cast<float*>(smem4) + plan_words<CoarsePlan>();
+  coarse_clear<DIM>(P, sm);
+  pdl_enter();
+  coarse_fetch_levels<DIM>(P, sm);
+  coarse_fetch(sm + P.lv[0].off[5], P.lv[0].r_glob, P.lv[0].cells);
+  cp_commit();
+  cp_wait<0>();
+  __syncthreads();
+  coarse_cycle<DIM>(P, sm);
+  const CoarseLevel& c0 = P.lv[0];
+  const float* x0 = sm + c0.off[4];
+  const int px = c0.n[0] + 2, pz = DIM == 3 ? px * (c0.n[1] + 2) : px;
+  const float inx = 1.0f / (float)c0.n[0], iny = 1.0f / (float)c0.n[1];
+  for (int c = threadIdx.x; c < c0.cells; c += blockDim.x) {
+    const int rest = __float2int_rz(((float)c + 0.5f) * inx);
+    const int k = DIM == 3 ? __float2int_rz(((float)rest + 0.5f) * iny) : rest;
+    const int j = DIM == 3 ? rest - k * c0.n[1] : 0;
+    c0.x_glob[c] = x0[(c - rest * c0.n[0] + 1) + (DIM == 3 ? px * (j + 1) : 0) + pz * (k + 1)];
+  }
 }
 
 // ------------------------------------------------------ hierarchy build
@@ -959,10 +1069,11 @@ size_t coarse_bytes(const MgHierarchy& H, int from) {
   return floats * sizeof(float);
 }
 
-CoarsePlan coarse_plan(const MgHierarchy& H, const MgWeights& W) {
+// The levels [from, ...) in one block.
+CoarsePlan coarse_plan(const MgHierarchy& H, const MgWeights& W, int from) {
   CoarsePlan P;
   std::memset(&P, 0, sizeof(P));
-  P.count = H.levels - H.coarse_from;
+  P.count = H.levels - from;
   P.nu = W.nu;
   P.sweeps = W.coarse_sweeps;
   int off = 0;
@@ -972,7 +1083,7 @@ CoarsePlan coarse_plan(const MgHierarchy& H, const MgWeights& W) {
     return o;
   };
   for (int q = 0; q < P.count; ++q) {
-    const MgLevel& M = H.L[H.coarse_from + q];
+    const MgLevel& M = H.L[from + q];
     CoarseLevel& c = P.lv[q];
     for (int a = 0; a < 3; ++a) c.n[a] = M.n[a];
     c.cells = (int)M.cells;
@@ -986,9 +1097,12 @@ CoarsePlan coarse_plan(const MgHierarchy& H, const MgWeights& W) {
     c.off[3] = take(c.cells);                          // isq
     c.off[4] = take(coarse_padded(H.dim, c.n));        // x (padded)
     c.off[5] = take(c.cells);                          // r
-    c.off[6] = take(coarse_padded(H.dim, c.n));        // res (padded)
-    P.K[q] = kern_of(W, H.coarse_from + q);
-    P.cw[q] = cw_of(W, H.coarse_from + q);
+    c.off[6] = take(coarse_padded(H.dim, c.n));        // u (padded)
+    c.dx = res::fast_div(c.n[0]);
+    c.dy = res::fast_div(c.n[1]);
+    c.warps = std::min(kCoarseThreads / 32, (c.cells + 31) / 32);
+    P.K[q] = kern_of(W, from + q);
+    P.cw[q] = cw_of(W, from + q);
   }
   return P;
 }
@@ -1285,6 +1399,55 @@ void level_sm(const MgLevel& M, const LV& LC, const Kern& K, bool first, const f
   }
 }
 
+#include "mg_cluster.cuh"
+
+// Levels of at most this many cells (below level 0) run in the cluster's one
+// launch instead of four grid kernels each.  An FCG iteration (us, before):
+// 300^2 64.4 (72.3), 512^2 74.9 (78.9), 1024^2 125.3 (131.5), 2048^2 250
+// (257), 80x48x48 96.0 (101), 100x75x61 134 (142), 256^3 752 (754).
+constexpr int64_t kTailCells = 32768;
+// Systems of at most this many cells run their whole FCG loop in a cluster
+// where it has the shared memory (2D to 256^2, 3D to about 36^3): 129^2 29.6
+// us an iteration (graph of grid kernels: 55.8), 256^2 42 (57.6), 12^3 21
+// (48), 24^3 37 (62), 33^3 56 (76).
+constexpr int64_t kFcgClusterCells = 65536;
+
+// Whether `fn` can run as a cluster of kMaxCluster blocks.
+template <class Fn>
+bool cluster_ok(Fn fn) {
+  return res::cluster_limit((const void*)fn, kClusterT) >= res::kMaxCluster;
+}
+
+// First level of the cluster's launch and its layout (words = 0: none).
+template <int DIM>
+int tail_from(const MgHierarchy& H, const MgWeights& W, ClusterLayout* C) {
+  for (int l = 1; l < H.coarse_from && cluster_ok(k_tail<DIM>); ++l) {
+    if (H.L[l].cells > kTailCells) continue;
+    *C = cluster_layout(H, W, l, false, H.L[l].r, H.L[l].x);
+    if (C->words > 0) return l;
+  }
+  return H.coarse_from;
+}
+
+template <typename... KArgs, typename... Args>
+void launch_in_cluster(void (*kernel)(KArgs...), size_t smem, cudaStream_t st, Args&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = res::kMaxCluster;
+  cfg.blockDim = kClusterT;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at[2];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = res::kMaxCluster;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[1].val.programmaticStreamSerializationAllowed = CFDB_PDL;
+  cfg.attrs = at;
+  cfg.numAttrs = 2;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
+  if (e != cudaSuccess && g_launch_error == cudaSuccess) g_launch_error = e;
+}
+
 // Enqueues z = M r (level-0 FP32 vectors) on `st`; returns the number of
 // kernels launched.
 template <int DIM>
@@ -1292,9 +1455,11 @@ int enqueue_cycle(const MgHierarchy& H, const MgWeights& W, const float* r0, flo
                   int64_t skip, const Hook* hook, cudaStream_t st) {
   int launches = 0;
   const int cf = H.coarse_from;
+  ClusterLayout CL;
+  const int tf = tail_from<DIM>(H, W, &CL);
   auto rp = [&](int l) -> const float* { return l == 0 ? r0 : H.L[l].r; };
   auto xp = [&](int l) -> float* { return l == 0 ? z0 : H.L[l].x; };
-  for (int l = 0; l < cf; ++l) {
+  for (int l = 0; l < tf; ++l) {
     const MgLevel& M = H.L[l];
     const LV LC = lv(H.L[l + 1]);
     const Kern K = kern_of(W, l);
@@ -1309,12 +1474,15 @@ int enqueue_cycle(const MgHierarchy& H, const MgWeights& W, const float* r0, flo
     level_res<DIM>(M, LC, xp(l), nullptr, 0.f, rp(l), nullptr, H.L[l + 1].r, sk, st);
     ++launches;
   }
-  if (cf < H.levels) {
-    const CoarsePlan P = coarse_plan(H, W);
-    launch(k_coarse<DIM>, 1, kCoarseThreads, H.coarse_smem, st, P);
+  if (tf < cf) {
+    launch_in_cluster(k_tail<DIM>, sizeof(float) * (size_t)CL.words, st, CL.P, CL.Q, CL.words);
+    ++launches;
+  } else if (cf < H.levels) {
+    const CoarsePlan P = coarse_plan(H, W, cf);
+    launch(k_coarse<DIM>, 1, kCoarseThreads, H.coarse_smem + sizeof(float) * plan_words<CoarsePlan>(), st, P);
     ++launches;
   }
-  for (int l = cf - 1; l >= 0; --l) {
+  for (int l = tf - 1; l >= 0; --l) {
     const MgLevel& M = H.L[l];
     const MgLevel& C = H.L[l + 1];
     const LV LC = lv(C);
@@ -1583,10 +1751,10 @@ cfdb_status mg_build(cfdb_context* ctx, MgHierarchy& H, const FineOperator& op) 
   // under a launch of this one
   if (op.dim == 2)
     CFDB_CUDA(ctx, cudaFuncSetAttribute(k_coarse<2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)kCoarseSmemCap));
+                                        (int)(kCoarseSmemCap + sizeof(float) * plan_words<CoarsePlan>())));
   else
     CFDB_CUDA(ctx, cudaFuncSetAttribute(k_coarse<3>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)kCoarseSmemCap));
+                                        (int)(kCoarseSmemCap + sizeof(float) * plan_words<CoarsePlan>())));
   return refresh_values(ctx, H, op);
 }
 
@@ -1646,6 +1814,8 @@ struct LearnedSolver {
 
 LearnedSolver* learned_create() {
   warm_quad_waves();
+  cluster_ok(k_tail<2>);  // opt-ins and queries, before any capture
+  cluster_ok(k_tail<3>);
   return new LearnedSolver();
 }
 
@@ -1757,6 +1927,47 @@ cfdb_status run_stream_mode(cfdb_context* ctx, LearnedSolver* s, const FineOpera
   return CFDB_OK;
 }
 
+void count_bytes(LearnedSolver* s, const FineOperator& op) {
+  // algorithmic bytes: the start (b, x in; r, r32 out) and per iteration the
+  // V-cycle, the direction pass (z, p_old, r in; p, q out), the update (x, p,
+  // r, q in; x, r, r32 out) and the z.q read of q; face arrays when present
+  int face_words = 0;
+  for (int a = 0; a < 3; ++a) face_words += op.full[a] ? 1 : 0;
+  const double n = (double)s->cells;
+  s->bytes_init = n * (8.0 * (3 + face_words) + 4.0);
+  s->bytes_iter = cycle_bytes(*s->H, s->W) + n * (4.0 + 8.0 * (4 + face_words)) +
+                  n * (8.0 * 6 + 4.0) + n * 8.0;
+}
+
+// The layout of a system's FCG in one cluster (words = 0: too large, no such
+// cluster, or the profilers' launch-by-launch mode).
+ClusterLayout fcg_layout(const LearnedSolver* s) {
+  const char* mode = std::getenv("CFDB_LEARNED_LAUNCH");
+  if (s->cells > kFcgClusterCells || (mode && std::strcmp(mode, "stream") == 0) ||
+      !(s->dim == 2 ? cluster_ok(k_fcg_cluster<2>) : cluster_ok(k_fcg_cluster<3>)))
+    return ClusterLayout{};
+  return cluster_layout(*s->H, s->W, 0, true, nullptr, nullptr);
+}
+
+cfdb_status run_in_cluster(cfdb_context* ctx, LearnedSolver* s, const FineOperator& op,
+                           const ClusterLayout& C) {
+  FcgArgs F;
+  std::memset(&F, 0, sizeof(F));
+  F.A = op.A;
+  F.S = s->S;
+  F.hist = s->hist;
+  F.hcap = s->hist_cap;
+  F.pin = op.pinned ? (int)op.ref : -1;
+  const size_t smem = sizeof(float) * (size_t)C.words;
+  const cudaError_t e =
+      s->dim == 2 ? res::launch_cluster(k_fcg_cluster<2>, res::kMaxCluster, res::kMaxCluster, kClusterT,
+                                        smem, ctx->stream, F, C.P, C.Q, C.words)
+                  : res::launch_cluster(k_fcg_cluster<3>, res::kMaxCluster, res::kMaxCluster, kClusterT,
+                                        smem, ctx->stream, F, C.P, C.Q, C.words);
+  if (e != cudaSuccess) return cuda_error(ctx, e, "learned solve in a cluster", __FILE__, __LINE__);
+  return CFDB_OK;
+}
+
 cfdb_status capture_graph(cfdb_context* ctx, LearnedSolver* s, const FineOperator& op) {
   s->free_graph();
   CFDB_CUDA(ctx, cudaGraphCreate(&s->graph, 0));
@@ -1796,15 +2007,6 @@ cfdb_status capture_graph(cfdb_context* ctx, LearnedSolver* s, const FineOperato
   CFDB_CUDA(ctx, cudaGraphInstantiate(&s->exec, s->graph, 0));
   s->launches_init = 1;
   s->launches_body = nv;
-  // algorithmic bytes: the start (b, x in; r, r32 out) and per iteration the
-  // V-cycle, the direction pass (z, p_old, r in; p, q out), the update (x, p,
-  // r, q in; x, r, r32 out) and the z.q read of q; face arrays when present
-  int face_words = 0;
-  for (int a = 0; a < 3; ++a) face_words += op.full[a] ? 1 : 0;
-  const double n = (double)s->cells;
-  s->bytes_init = n * (8.0 * (3 + face_words) + 4.0);
-  s->bytes_iter = cycle_bytes(*s->H, s->W) + n * (4.0 + 8.0 * (4 + face_words)) +
-                  n * (8.0 * 6 + 4.0) + n * 8.0;
   return CFDB_OK;
 }
 
@@ -1889,7 +2091,6 @@ cfdb_status learned_solve(cfdb_context* ctx, LearnedSolver* s, const FineOperato
     cfdb_status st = ensure_state(ctx, s, op, version, &recapture);
     if (st != CFDB_OK) return st;
   }
-  if (!s->exec) recapture = true;
   const int64_t want_hist = std::max<int64_t>(hist_cap, 1);
   if (s->hist_cap < want_hist) {
     cudaFree(s->hist);
@@ -1904,13 +2105,17 @@ cfdb_status learned_solve(cfdb_context* ctx, LearnedSolver* s, const FineOperato
     s->have_w = true;
     recapture = true;
   }
-  if (recapture || !s->exec) {
+  const ClusterLayout CL = fcg_layout(s);
+  const bool in_cluster = CL.words > 0;
+  if (recapture) s->free_graph();
+  if (!in_cluster && !s->exec) {
     cfdb_status st = capture_graph(ctx, s, op);
     if (st != CFDB_OK) {
       s->free_graph();
       return st;
     }
   }
+  count_bytes(s, op);
   FcgState& hs = *s->S_host;
   std::memset(&hs, 0, sizeof(hs));
   hs.b = b;
@@ -1923,7 +2128,10 @@ cfdb_status learned_solve(cfdb_context* ctx, LearnedSolver* s, const FineOperato
   CFDB_CUDA(ctx, cudaMemcpyAsync(s->S, &hs, sizeof(FcgState), cudaMemcpyHostToDevice, ctx->stream));
   CFDB_CUDA(ctx, cudaEventRecord(ctx->ev_k0, ctx->stream));
   const char* mode = std::getenv("CFDB_LEARNED_LAUNCH");
-  if (mode && std::strcmp(mode, "stream") == 0) {
+  if (in_cluster) {
+    cfdb_status st = run_in_cluster(ctx, s, op, CL);
+    if (st != CFDB_OK) return st;
+  } else if (mode && std::strcmp(mode, "stream") == 0) {
     cfdb_status st = run_stream_mode(ctx, s, op);
     if (st != CFDB_OK) return st;
   } else {
@@ -1940,7 +2148,7 @@ cfdb_status learned_solve(cfdb_context* ctx, LearnedSolver* s, const FineOperato
   out->final_residual = hs.res;
   out->kernel_ms = ms;
   out->bytes = s->bytes_init + s->bytes_iter * (double)hs.it;
-  out->launches = s->launches_init + s->launches_body * hs.it;
+  out->launches = in_cluster ? 1 : s->launches_init + s->launches_body * hs.it;
   count_launch(ctx, (int)std::min<int64_t>(out->launches, 1 << 30));
   return CFDB_OK;
 }

@@ -169,7 +169,9 @@ def _face_op(ctx, dim, n, seed):
     return op, MO.hierarchy(dims, f, dim)
 
 
-@pytest.mark.parametrize("dim,n", [(2, (40, 36)), (3, (24, 20, 18))])
+# the last four: levels below the first run in one thread-block cluster
+@pytest.mark.parametrize("dim,n", [(2, (40, 36)), (3, (24, 20, 18)), (2, (200, 150)), (2, (301, 163)),
+                                   (3, (50, 41, 37)), (3, (39, 44, 70))])
 def test_vcycle_kernels_match_oracle(ctx, dim, n):
     """One application of the solve's tiled V-cycle (grid levels + the
     block-resident coarse levels) against the FP64 restatement."""

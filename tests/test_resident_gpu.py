@@ -129,3 +129,31 @@ def test_band_solves_match_oracle(ctx, n, method, jacobi):
     assert got.status == ref.status and got.iterations == ref.iterations
     np.testing.assert_allclose(got.residual_history, ref.history, rtol=1e-8)
     assert _rel(got.solution, ref.solution) <= 1e-10
+
+
+# grids at the edges of the learned solve's cluster form: one block with all
+# planes, fewer planes than blocks, partial last blocks, odd coarsenings, the
+# largest that fit, and (the last of each dimension) ones that do not
+@pytest.mark.parametrize("n", [(8, 8), (17, 5), (31, 129), (129, 31), (96, 90), (255, 257), (301, 290),
+                               (5, 6, 7), (9, 24, 37), (33, 33, 33), (24, 30, 9), (41, 40, 39)])
+@pytest.mark.parametrize("outlet", [True, False])
+def test_learned_solve_matches_jacobi(ctx, n, outlet):
+    """The learned FCG and the Jacobi-CG of one system, both to a relative residual of 1e-12:
+    the solutions agree within 1e-9 with an outlet (the FP64 parity bar), 1e-7 in a closed
+    domain, whose nearly free constant mode the residual sees 10^4 times less."""
+    from cfdapp_b200.cfdb import LinearSolverSettings, POperator
+    case, fc, diag, off, rhs = _system(n, 9, outlet)
+    ref_cell = 0 if outlet else case.cells() // 2
+    if not outlet:
+        rhs = rhs - rhs.mean()
+        rhs[ref_cell] = 0.0
+    op = POperator(ctx, len(n), n, tuple(float(m) for m in n), face_coeff=fc, pinned=not outlet,
+                   reference_cell=ref_cell)
+    got = {}
+    for pc in ("jacobi", "learned_mg"):
+        got[pc] = op.solve(rhs, LinearSolverSettings(absolute_tolerance=0.0, preconditioner=pc,
+                                                     relative_tolerance=1e-12, max_iterations=20000))
+        assert got[pc].status == "Converged"
+        assert got[pc].fallback_iterations == 0
+    assert got["learned_mg"].iterations <= got["jacobi"].iterations
+    assert _rel(got["learned_mg"].solution, got["jacobi"].solution) <= (1e-9 if outlet else 1e-7)
