@@ -282,3 +282,18 @@ def test_learned_beats_jacobi_on_a_harvested_2048_cavity_system(ctx):
     assert learned.fallback_iterations == 0
     assert learned.true_residual / learned.initial_residual <= 1e-8
     assert jac.device_ms >= 3.0 * learned.device_ms, (jac.device_ms, learned.device_ms)
+
+
+@pytest.mark.parametrize("dim,n,samples", [(2, (256, 250), 70), (3, (11, 9, 10), 3), (2, (33, 20), 1)])
+def test_loss_and_gradient_are_the_mean_over_samples(ctx, dim, n, samples):
+    """A step over many samples (70 at 256x250 go in two chunks of the scratch) against the
+    same samples one at a time: each sample's arithmetic is the same, only the FP64 sums over
+    cells and samples are added in another order (1e-10 of the largest gradient)."""
+    op, _ = _face_op(ctx, dim, n, 41)
+    e = np.random.default_rng(42).normal(size=(samples, int(np.prod(n)))).astype(np.float32)
+    loss, gk, gc = op.mg_loss_grad(e)
+    one = [op.mg_loss_grad(v) for v in e]
+    assert loss == pytest.approx(np.mean([o[0] for o in one]), rel=1e-12)
+    for got, ref in ((gk, np.mean([o[1] for o in one], axis=0)),
+                     (gc, np.mean([o[2] for o in one], axis=0))):
+        np.testing.assert_allclose(got, ref, rtol=0, atol=1e-10 * np.abs(ref).max())
