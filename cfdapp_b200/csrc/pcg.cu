@@ -712,6 +712,11 @@ cfdb_status check_finite(cfdb_context* ctx, const double* v, int64_t n, bool* ok
   return CFDB_OK;
 }
 
+// Whether the operator's PCG runs on chip (vectors of `word` bytes).
+bool on_chip(const cfdb_context* ctx, const cfdb_poperator* op, size_t word) {
+  return resident_pcg_fits(ctx, op->knx, op->kny, op->knz, word);
+}
+
 // Plain FP64 PCG on device vectors.
 cfdb_status solve_fp64(cfdb_context* ctx, cfdb_poperator* op, const cfdb_linear_settings* s,
                        const double* b, double* x, bool x0_zero, int64_t hist_cap,
@@ -719,7 +724,7 @@ cfdb_status solve_fp64(cfdb_context* ctx, cfdb_poperator* op, const cfdb_linear_
   const int64_t n = op->cells;
   // on chip where it fits: the exchanged values (w64[1]) and the inverse
   // diagonal of a table operator (w64[6]) are its only vectors in memory
-  const bool chip = resident_pcg_fits(ctx, view<double>(op));
+  const bool chip = on_chip(ctx, op, sizeof(double));
   for (int q : {0, 1, 2, 6}) {
     if (chip && q != 1 && (q != 6 || op->invd64)) continue;
     cfdb_status st = alloc_vec(ctx, &op->w64[q], n);
@@ -729,8 +734,8 @@ cfdb_status solve_fp64(cfdb_context* ctx, cfdb_poperator* op, const cfdb_linear_
   if (st != CFDB_OK) return st;
   if (chip)
     st = resident_pcg(ctx, view<double>(op), op->grid.dim, op->invd64, b, x, op->w64[1],
-                      op->invd64 ? nullptr : op->w64[6], s->abs_tol, s->rel_tol,
-                      s->max_iterations, op->hist_dev, hist_cap);
+                      op->invd64 ? nullptr : op->w64[6],
+                      ResidentLimits{s->abs_tol, s->rel_tol, s->max_iterations, op->hist_dev, hist_cap, 0.0, 0});
   else
     st = run_pcg<double>(ctx, op, b, x, op->w64[0], op->w64[1], op->w64[2], op->w64[6], x0_zero ? 1 : 0,
                          s->abs_tol, s->rel_tol, s->max_iterations, op->hist_dev, hist_cap);
@@ -751,17 +756,25 @@ cfdb_status solve_mixed(cfdb_context* ctx, cfdb_poperator* op, const cfdb_linear
                         const double* b, double* x, int64_t hist_cap,
                         cfdb_linear_result* res) {
   const int64_t n = op->cells;
-  for (int q : {1, 2, 5}) {
-    cfdb_status st = alloc_vec(ctx, &op->w32[q], n);
-    if (st != CFDB_OK) return st;
-  }
-  cfdb_status st = alloc_vec(ctx, &op->w64[0], n);
-  if (st != CFDB_OK) return st;
-  st = ensure_hist(ctx, op, std::max<int64_t>(hist_cap, 1));
-  if (st != CFDB_OK) return st;
   const double delta = s->inner_rel_tol > 0.0 ? s->inner_rel_tol : 0.1;
-  st = run_pcg_mixed(ctx, op, b, x, op->w64[0], op->w32[1], op->w32[2], op->w32[5], 0, s->abs_tol,
-                     s->rel_tol, s->max_iterations, delta, op->hist_dev, hist_cap);
+  cfdb_status st = ensure_hist(ctx, op, std::max<int64_t>(hist_cap, 1));
+  if (st != CFDB_OK) return st;
+  if (on_chip(ctx, op, sizeof(double))) {
+    for (int q : {1, 6}) {
+      if (q == 6 && op->invd64) continue;
+      if ((st = alloc_vec(ctx, &op->w64[q], n)) != CFDB_OK) return st;
+    }
+    st = resident_pcg(ctx, view<double>(op), op->grid.dim, op->invd64, b, x, op->w64[1],
+                      op->invd64 ? nullptr : op->w64[6],
+                      ResidentLimits{s->abs_tol, s->rel_tol, s->max_iterations, op->hist_dev, hist_cap,
+                                     delta, OUT_REPLACEMENTS});
+  } else {
+    for (int q : {1, 2, 5})
+      if ((st = alloc_vec(ctx, &op->w32[q], n)) != CFDB_OK) return st;
+    if ((st = alloc_vec(ctx, &op->w64[0], n)) != CFDB_OK) return st;
+    st = run_pcg_mixed(ctx, op, b, x, op->w64[0], op->w32[1], op->w32[2], op->w32[5], 0, s->abs_tol,
+                       s->rel_tol, s->max_iterations, delta, op->hist_dev, hist_cap);
+  }
   if (st != CFDB_OK) return st;
   st = read_scalars(ctx, 8);
   if (st != CFDB_OK) return st;
@@ -823,8 +836,13 @@ cfdb_status solve_refined(cfdb_context* ctx, cfdb_poperator* op, const cfdb_line
     // inner: A e = r32 from e = 0 in FP32, reduction inner_tol
     const int64_t budget = s->max_iterations - inner_total;
     CFDB_CUDA(ctx, cudaMemsetAsync(e32, 0, sizeof(float) * (size_t)n, ctx->stream));
-    st = run_pcg<float>(ctx, op, b32, e32, r32, op->w32[1], op->w32[2], op->w32[5], 1, 0.0, inner_tol,
-                        budget, op->hist_dev, 0);
+    if (on_chip(ctx, op, sizeof(float)))
+      st = resident_pcg(ctx, view<float>(op), op->grid.dim, op->invd32, b32, e32, op->w32[1],
+                        op->invd32 ? nullptr : op->w32[5],
+                        ResidentLimits{0.0, inner_tol, budget, op->hist_dev, 0, 0.0, 0});
+    else
+      st = run_pcg<float>(ctx, op, b32, e32, r32, op->w32[1], op->w32[2], op->w32[5], 1, 0.0, inner_tol,
+                          budget, op->hist_dev, 0);
     if (st != CFDB_OK) return st;
     st = read_scalars(ctx, 8);
     if (st != CFDB_OK) return st;

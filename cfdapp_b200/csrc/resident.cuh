@@ -60,26 +60,29 @@ __host__ __device__ inline FastDiv fast_div(uint32_t d) {
 
 // Couplings of one cell to its neighbours (0 across the domain's edge), its
 // diagonal and the preconditioner's inverse diagonal.
+template <typename V>
 struct Cf {
-  double xl, xh, yl, yh, zl, zh, dg, inv;
+  V xl, xh, yl, yh, zl, zh, dg, inv;
 };
 
 // ------------------------------------------------------------------ operators
 //
 // An operator has the extents of kernel space (a 2D grid is nx x 1 x ny),
-// load() -> Cf of a cell and mul() -> the row's product.
+// load() -> Cf of a cell and mul() -> the row's product; V is the type of its
+// vectors and coefficients.
 
 // The p' operator (poperator.cuh), tables or face arrays; Jacobi.
-template <int DIM>
+template <int DIM, typename T = double>
 struct FaceOp {
   static constexpr int kDim = DIM;
-  OpView<double> A;
-  const double* invd;  // 1/diag of face-array operators, or null
+  using V = T;
+  OpView<V> A;
+  const V* invd;  // 1/diag of face-array operators, or null
   int nx, ny, nz;
   uint32_t sz;
   FastDiv dx, dy;
-  __device__ __forceinline__ Cf load(uint32_t c, int i, int j, int k) const {
-    Cf f;
+  __device__ __forceinline__ Cf<V> load(uint32_t c, int i, int j, int k) const {
+    Cf<V> f;
     const uint32_t row = (uint32_t)j + (uint32_t)ny * k;
     if (A.fx) {
       f.xl = __ldg(A.fx + c + row);
@@ -88,7 +91,7 @@ struct FaceOp {
       f.xl = __ldg(A.tx + i);
       f.xh = __ldg(A.tx + i + 1);
     }
-    f.yl = f.yh = 0.0;
+    f.yl = f.yh = V(0);
     if (DIM == 3) {
       if (A.fy) {
         f.yl = __ldg(A.fy + c + (uint32_t)nx * k);
@@ -106,33 +109,32 @@ struct FaceOp {
       f.zh = __ldg(A.tz + k + 1);
     }
     if (A.pinned && c == (uint32_t)A.ref) {
-      f.xl = f.xh = f.yl = f.yh = f.zl = f.zh = 0.0;
-      f.dg = f.inv = 1.0;
+      f.xl = f.xh = f.yl = f.yh = f.zl = f.zh = V(0);
+      f.dg = f.inv = V(1);
       return f;
     }
     // the reference's face order (poperator.cuh load_coef)
     f.dg = ((((f.xl + f.xh) + f.yl) + f.yh) + f.zl) + f.zh;
     f.inv = invd ? __ldg(invd + c) : rcp_rn(f.dg);
-    if (i == 0) f.xl = 0.0;
-    if (i == nx - 1) f.xh = 0.0;
-    if (j == 0) f.yl = 0.0;
-    if (j == ny - 1) f.yh = 0.0;
-    if (k == 0) f.zl = 0.0;
-    if (k == nz - 1) f.zh = 0.0;
+    if (i == 0) f.xl = V(0);
+    if (i == nx - 1) f.xh = V(0);
+    if (j == 0) f.yl = V(0);
+    if (j == ny - 1) f.yh = V(0);
+    if (k == 0) f.zl = V(0);
+    if (k == nz - 1) f.zh = V(0);
     return f;
   }
   // the preconditioner's inverse diagonal alone
-  __device__ __forceinline__ double inverse(uint32_t c, int i, int j, int k) const {
+  __device__ __forceinline__ V inverse(uint32_t c, int i, int j, int k) const {
     if (invd) return __ldg(invd + c);
     if (A.fx || A.fy || A.fz) return load(c, i, j, k).inv;
-    if (A.pinned && c == (uint32_t)A.ref) return 1.0;
-    double d = __ldg(A.tx + i) + __ldg(A.tx + i + 1);
+    if (A.pinned && c == (uint32_t)A.ref) return V(1);
+    V d = __ldg(A.tx + i) + __ldg(A.tx + i + 1);
     if (DIM == 3) d = (d + __ldg(A.ty + j)) + __ldg(A.ty + j + 1);
     return rcp_rn((d + __ldg(A.tz + k)) + __ldg(A.tz + k + 1));
   }
-  __device__ __forceinline__ double mul(const Cf& f, double v, double w, double e, double s,
-                                        double n, double b, double t) const {
-    double off = f.xl * w;
+  __device__ __forceinline__ V mul(const Cf<V>& f, V v, V w, V e, V s, V n, V b, V t) const {
+    V off = f.xl * w;
     off = fma(f.xh, e, off);
     if (DIM == 3) {
       off = fma(f.yl, s, off);
@@ -149,14 +151,15 @@ struct FaceOp {
 template <int DIM>
 struct BandOp {
   static constexpr int kDim = DIM;
+  using V = double;
   const double* diag;
   const double *oxl, *oxh, *oyl, *oyh, *ozl, *ozh;
   const double* pinv;
   int nx, ny, nz;
   uint32_t sz;
   FastDiv dx, dy;
-  __device__ __forceinline__ Cf load(uint32_t c, int i, int j, int k) const {
-    Cf f;
+  __device__ __forceinline__ Cf<double> load(uint32_t c, int i, int j, int k) const {
+    Cf<double> f;
     f.xl = i > 0 ? __ldg(oxl + c) : 0.0;
     f.xh = i < nx - 1 ? __ldg(oxh + c) : 0.0;
     f.yl = DIM == 3 && j > 0 ? __ldg(oyl + c) : 0.0;
@@ -171,7 +174,7 @@ struct BandOp {
     return pinv ? __ldg(pinv + c) : 1.0;
   }
   // ascending column order of the reference's CSR rows
-  __device__ __forceinline__ double mul(const Cf& f, double v, double w, double e, double s,
+  __device__ __forceinline__ double mul(const Cf<double>& f, double v, double w, double e, double s,
                                         double n, double b, double t) const {
     double sum = f.zl * b;
     if (DIM == 3) sum += f.yl * s;
@@ -295,6 +298,15 @@ struct ClusterTeam {
     return true;
   }
   // vec[c] of a cell outside this block's range (vec: this block's shared array)
+  __device__ __forceinline__ float remote(const float* vec, const float*, uint32_t c) const {
+    const uint32_t r = dlen.div(c);
+    const uint32_t a = (uint32_t)__cvta_generic_to_shared(vec + (c - r * len));
+    uint32_t ra;
+    float out;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(a), "r"(r));
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(out) : "r"(ra) : "memory");
+    return out;
+  }
   __device__ __forceinline__ double remote(const double* vec, const double*, uint32_t c) const {
     const uint32_t r = dlen.div(c);
     const uint32_t a = (uint32_t)__cvta_generic_to_shared(vec + (c - r * len));
@@ -383,25 +395,30 @@ struct GridTeam {
     }
     return true;
   }
-  __device__ __forceinline__ double remote(const double*, const double* pub, uint32_t c) const {
+  template <typename V>
+  __device__ __forceinline__ V remote(const V*, const V* pub, uint32_t c) const {
     return __ldcg(pub + c);
   }
 };
 
 // ------------------------------------------------------------------- routines
 
-struct Io {
-  const double* b;
-  double* x;
-  double* pub;   // GridTeam: published values (cells), else null
-  double* pub2;  // GridTeam, BiCGSTAB: published s (cells)
-  double* inv;   // scratch (cells) for M^-1 of a table operator, or null
+template <typename V>
+struct IoT {
+  const V* b;
+  V* x;
+  V* pub;   // GridTeam: published values (cells), else null
+  V* pub2;  // GridTeam, BiCGSTAB: published s (cells)
+  V* inv;   // scratch (cells) for M^-1 of a table operator, or null
   double abs_tol, rel_tol;
   int64_t max_it;
   double* hist;
   int64_t hist_cap;
-  double* out;  // status, iterations, initial residual, final residual, restarts
+  double* out;   // status, iterations, initial residual, final residual, restarts
+  double delta;  // MIXED: drop of the residual between replacements
+  double* reps;  // MIXED: where the number of replacements goes
 };
+using Io = IoT<double>;
 
 // Range of cells of block `rank`: [rank len, min(n, (rank + 1) len)).
 struct Range {
@@ -416,7 +433,8 @@ __device__ __forceinline__ Range range_of(uint32_t n, uint32_t len, int rank) {
 // solve when there are few of them, else loaded again where they are used.
 template <class Op, int NC, bool PRE>
 struct Cells {
-  Cf f[PRE ? NC : 1];
+  using V = typename Op::V;
+  Cf<V> f[PRE ? NC : 1];
   __device__ __forceinline__ void ijk(const Op& A, uint32_t c, int& i, int& j, int& k) const {
     const uint32_t row = A.dx.div(c);
     i = (int)(c - row * (uint32_t)A.nx);
@@ -429,7 +447,7 @@ struct Cells {
       j = 0;
     }
   }
-  __device__ __forceinline__ Cf load(const Op& A, uint32_t c) const {
+  __device__ __forceinline__ Cf<V> load(const Op& A, uint32_t c) const {
     int i, j, k;
     ijk(A, c, i, j, k);
     return A.load(c, i, j, k);
@@ -444,11 +462,11 @@ struct Cells {
       }
     }
   }
-  __device__ __forceinline__ Cf at(const Op& A, int q, uint32_t c) const {
+  __device__ __forceinline__ Cf<V> at(const Op& A, int q, uint32_t c) const {
     if constexpr (PRE) return f[q];
     else return load(A, c);
   }
-  __device__ __forceinline__ double inverse(const Op& A, int q, uint32_t c) const {
+  __device__ __forceinline__ V inverse(const Op& A, int q, uint32_t c) const {
     if constexpr (PRE) return f[q].inv;
     int i, j, k;
     ijk(A, c, i, j, k);
@@ -460,35 +478,33 @@ struct Cells {
 // the array.  Else x- and y-neighbours past the range's ends are read from
 // the published vector (couplings of 0 read nothing), and the z-neighbours'
 // values come with the call.
-template <bool HALO, class Op, class Team>
-__device__ __forceinline__ double apply(const Op& A, const Team& T, const Cf& f, const Range& R,
-                                        uint32_t lc, const double* vec, const double* pub,
-                                        double zlo, double zhi) {
+template <bool HALO, class Op, class Team, typename V = typename Op::V>
+__device__ __forceinline__ V apply(const Op& A, const Team& T, const Cf<V>& f, const Range& R,
+                                   uint32_t lc, const V* vec, const V* pub, V zlo, V zhi) {
   const int sy = A.nx, sz = (int)A.sz;
-  const double* v = vec + lc;
+  const V* v = vec + lc;
   if constexpr (HALO) {
-    return A.mul(f, v[0], v[-1], v[1], Op::kDim == 3 ? v[-sy] : 0.0, Op::kDim == 3 ? v[sy] : 0.0,
+    return A.mul(f, v[0], v[-1], v[1], Op::kDim == 3 ? v[-sy] : V(0), Op::kDim == 3 ? v[sy] : V(0),
                  v[-sz], v[sz]);
   } else {
     const uint32_t c = R.c0 + lc;
-    auto get = [&](double coupling, int off) -> double {
+    auto get = [&](V coupling, int off) -> V {
       const uint32_t li = lc + (uint32_t)off;  // wraps below 0: past count
       if (li < R.count) return vec[li];
-      return coupling == 0.0 ? 0.0 : T.remote(vec, pub, c + (uint32_t)off);
+      return coupling == V(0) ? V(0) : T.remote(vec, pub, c + (uint32_t)off);
     };
-    return A.mul(f, v[0], get(f.xl, -1), get(f.xh, 1), Op::kDim == 3 ? get(f.yl, -sy) : 0.0,
-                 Op::kDim == 3 ? get(f.yh, sy) : 0.0, zlo, zhi);
+    return A.mul(f, v[0], get(f.xl, -1), get(f.xh, 1), Op::kDim == 3 ? get(f.yl, -sy) : V(0),
+                 Op::kDim == 3 ? get(f.yh, sy) : V(0), zlo, zhi);
   }
 }
 
 // (A x)(c) with x in global memory.
-template <class Op>
-__device__ __forceinline__ double apply_global(const Op& A, const Cf& f, uint32_t c,
-                                               const double* x) {
-  auto get = [&](double coupling, uint32_t at) { return coupling == 0.0 ? 0.0 : __ldcg(x + at); };
+template <class Op, typename V = typename Op::V>
+__device__ __forceinline__ V apply_global(const Op& A, const Cf<V>& f, uint32_t c, const V* x) {
+  auto get = [&](V coupling, uint32_t at) { return coupling == V(0) ? V(0) : __ldcg(x + at); };
   const uint32_t sy = (uint32_t)A.nx, sz = A.sz;
   return A.mul(f, __ldcg(x + c), get(f.xl, c - 1), get(f.xh, c + 1),
-               Op::kDim == 3 ? get(f.yl, c - sy) : 0.0, Op::kDim == 3 ? get(f.yh, c + sy) : 0.0,
+               Op::kDim == 3 ? get(f.yl, c - sy) : V(0), Op::kDim == 3 ? get(f.yh, c + sy) : V(0),
                get(f.zl, c - sz), get(f.zh, c + sz));
 }
 
@@ -500,47 +516,78 @@ __device__ __forceinline__ double apply_global(const Op& A, const Cf& f, uint32_
 // (the two reductions).  Otherwise (3D grids whose planes are larger than
 // shared memory allows) p itself is published, which takes a third.
 //
-// Shared memory (doubles): p (len, HALO: + 2 H), r (len), ClusterTeam: z
+// MIXED (V = double): the mixed-precision solve of pcg_tma.cuh -- z and p are
+// rounded to FP32 as they are formed, x and r stay FP64 and r is replaced by
+// b - A x when it has fallen by P.delta, when it meets the tolerance and at
+// the iteration cap.
+//
+// Shared memory (words of V): p (len, HALO: + 2 H), r (len), ClusterTeam: z
 // (len), XS: x (len).
-template <int T, int NC, bool PRE, bool XS, bool HALO, class Op, class Team>
-__device__ __forceinline__ void cg_run(const Op& A, uint32_t n, uint32_t len, const Io& P,
-                                       Team& team, double* sm) {
+template <int T, int NC, bool PRE, bool XS, bool HALO, bool MIXED = false, class Op, class Team,
+          typename V = typename Op::V>
+__device__ __forceinline__ void cg_run(const Op& A, uint32_t n, uint32_t len, const IoT<V>& P,
+                                       Team& team, V* sm) {
   static_assert(HALO || Team::kGlobal, "a cluster's planes fit its shared memory");
   const Range R = range_of(n, len, team.rank());
   const uint32_t H = A.sz;  // reach of the stencil
-  double* p = HALO ? sm + H : sm;
-  double* r = sm + len + (HALO ? 2 * H : 0);
-  double* zs = r + len;
-  double* xs = zs + (Team::kGlobal ? 0 : len);
+  V* p = HALO ? sm + H : sm;
+  V* r = sm + len + (HALO ? 2 * H : 0);
+  V* zs = r + len;
+  V* xs = zs + (Team::kGlobal ? 0 : len);
   const bool leader = team.rank() == 0 && threadIdx.x == 0;
   Cells<Op, NC, PRE> cells;
   cells.template init<T>(A, R);
   if (HALO)
-    for (uint32_t q = threadIdx.x; q < len + 2 * H; q += T) sm[q] = 0.0;
-  double z[NC];  // z = M^-1 r between the sweeps, q = A p within an iteration
+    for (uint32_t q = threadIdx.x; q < len + 2 * H; q += T) sm[q] = V(0);
+  V z[NC];  // z = M^-1 r between the sweeps, q = A p within an iteration
   // z of a cell for the blocks whose stencils reach it
-  auto publish = [&](uint32_t lc, double v) {
+  auto rounded = [](V v) { return MIXED ? (V)(float)v : v; };
+  // p = z + beta p_old
+  auto direction = [](V beta, V old, V zv) {
+    return MIXED ? (V)fmaf((float)beta, (float)old, (float)zv) : fma(beta, old, zv);
+  };
+  auto publish = [&](uint32_t lc, V v) {
     if (!Team::kGlobal) zs[lc] = v;
     else if (!HALO || lc < H || lc + H >= R.count) P.pub[R.c0 + lc] = v;
   };
-  double acc[2] = {0.0, 0.0};
+  // r = b - A x (x in global memory), z = M^-1 r; r.r, r.z
+  auto residual = [&](double (&acc)[2]) -> bool {
+    acc[0] = acc[1] = 0.0;
 #pragma unroll
-  for (int q = 0; q < NC; ++q) {
-    const uint32_t lc = threadIdx.x + q * T;
-    if (lc < R.count) {
-      const uint32_t c = R.c0 + lc;
-      const Cf f = cells.at(A, q, c);
-      const double rn = __ldg(P.b + c) - apply_global(A, f, c, P.x);
-      r[lc] = rn;
-      if (XS) xs[lc] = __ldcg(P.x + c);
-      z[q] = f.inv * rn;
-      if (HALO) publish(lc, z[q]);
-      if (!PRE && P.inv) P.inv[c] = f.inv;
-      acc[0] += rn * rn;
-      acc[1] += rn * z[q];
+    for (int q = 0; q < NC; ++q) {
+      const uint32_t lc = threadIdx.x + q * T;
+      if (lc < R.count) {
+        const uint32_t c = R.c0 + lc;
+        const Cf<V> f = cells.at(A, q, c);
+        const V rn = __ldg(P.b + c) - apply_global(A, f, c, P.x);
+        r[lc] = rn;
+        z[q] = rounded(f.inv * rn);
+        if (HALO) publish(lc, z[q]);
+        if (!PRE && P.inv) P.inv[c] = f.inv;
+        acc[0] += (double)rn * (double)rn;
+        acc[1] += (double)rn * (double)z[q];
+      }
+    }
+    return team.reduce(acc);
+  };
+  auto flush_x = [&]() {
+    if (XS) {
+#pragma unroll
+      for (int q = 0; q < NC; ++q) {
+        const uint32_t lc = threadIdx.x + q * T;
+        if (lc < R.count) P.x[R.c0 + lc] = xs[lc];
+      }
+    }
+  };
+  double acc[2];
+  if (XS) {
+#pragma unroll
+    for (int q = 0; q < NC; ++q) {
+      const uint32_t lc = threadIdx.x + q * T;
+      if (lc < R.count) xs[lc] = __ldcg(P.x + R.c0 + lc);
     }
   }
-  if (!team.reduce(acc)) return;
+  if (!residual(acc)) return;
   const double b0 = sqrt(acc[0]);
   double rz = acc[1];
   auto conv = [&](double res) {
@@ -552,37 +599,33 @@ __device__ __forceinline__ void cg_run(const Op& A, uint32_t n, uint32_t len, co
       P.out[1] = (double)it;
       P.out[3] = fin;
     }
-    if (XS && it > 0) {
-#pragma unroll
-      for (int q = 0; q < NC; ++q) {
-        const uint32_t lc = threadIdx.x + q * T;
-        if (lc < R.count) P.x[R.c0 + lc] = xs[lc];
-      }
-    }
+    if (it > 0) flush_x();
   };
   if (leader) {
     P.out[2] = b0;
     P.out[4] = 0.0;
+    if (MIXED) *P.reps = 0.0;
     if (P.hist_cap > 0) P.hist[0] = b0;
   }
   if (b0 == 0.0 || conv(b0)) return finish(CFDB_SOLVER_CONVERGED, 0, b0);
   if (!isfinite(rz)) return finish(CFDB_SOLVER_BREAKDOWN, 0, b0);
   // cells of the halo inside the domain: [lo0, c0) and [c0 + count, hi1)
   const uint32_t lo = min(H, R.c0), hi = min(H, n - (R.c0 + R.count));
-  double res_cur = b0, beta = 0.0;
+  double res_cur = b0, beta = 0.0, replaced = b0;
+  int64_t reps = 0;
   for (int64_t it = 1; it <= P.max_it; ++it) {
     // p = z + beta p
     if (HALO && R.count > 0) {
       for (uint32_t h = threadIdx.x; h < lo + hi; h += T) {
         const int at = h < lo ? -(int)(lo - h) : (int)(R.count + (h - lo));
-        p[at] = fma(beta, p[at], team.remote(zs, P.pub, R.c0 + (uint32_t)at));
+        p[at] = direction((V)beta, p[at], team.remote(zs, P.pub, R.c0 + (uint32_t)at));
       }
     }
 #pragma unroll
     for (int q = 0; q < NC; ++q) {
       const uint32_t lc = threadIdx.x + q * T;
       if (lc < R.count) {
-        const double v = it == 1 ? z[q] : fma(beta, p[lc], z[q]);
+        const V v = it == 1 ? z[q] : direction((V)beta, p[lc], z[q]);
         p[lc] = v;
         if (!HALO) publish(lc, v);
       }
@@ -595,9 +638,9 @@ __device__ __forceinline__ void cg_run(const Op& A, uint32_t n, uint32_t len, co
       for (int q = 0; q < NC; ++q) {
         const uint32_t lc = threadIdx.x + q * T;
         if (lc < R.count) {
-          const Cf f = cells.at(A, q, R.c0 + lc);
-          z[q] = apply<true>(A, team, f, R, lc, p, P.pub, 0.0, 0.0);
-          pap[0] += p[lc] * z[q];
+          const Cf<V> f = cells.at(A, q, R.c0 + lc);
+          z[q] = apply<true>(A, team, f, R, lc, p, P.pub, V(0), V(0));
+          pap[0] += (double)p[lc] * (double)z[q];
         }
       }
     } else {
@@ -606,22 +649,22 @@ __device__ __forceinline__ void cg_run(const Op& A, uint32_t n, uint32_t len, co
       constexpr int G = NC % 4 == 0 ? 4 : (NC % 2 == 0 ? 2 : 1);
 #pragma unroll
       for (int g = 0; g < NC; g += G) {
-        double lo_z[G], hi_z[G];
+        V lo_z[G], hi_z[G];
 #pragma unroll
         for (int u = 0; u < G; ++u) {
           const uint32_t c = R.c0 + threadIdx.x + (g + u) * T;
           const bool in = threadIdx.x + (g + u) * T < R.count;
-          lo_z[u] = in && c >= H ? __ldcg(P.pub + (c - H)) : 0.0;
-          hi_z[u] = in && c + H < n ? __ldcg(P.pub + (c + H)) : 0.0;
+          lo_z[u] = in && c >= H ? __ldcg(P.pub + (c - H)) : V(0);
+          hi_z[u] = in && c + H < n ? __ldcg(P.pub + (c + H)) : V(0);
         }
 #pragma unroll
         for (int u = 0; u < G; ++u) {
           const int q = g + u;
           const uint32_t lc = threadIdx.x + q * T;
           if (lc < R.count) {
-            const Cf f = cells.at(A, q, R.c0 + lc);
+            const Cf<V> f = cells.at(A, q, R.c0 + lc);
             z[q] = apply<false>(A, team, f, R, lc, p, P.pub, lo_z[u], hi_z[u]);
-            pap[0] += p[lc] * z[q];
+            pap[0] += (double)p[lc] * (double)z[q];
           }
         }
       }
@@ -636,18 +679,26 @@ __device__ __forceinline__ void cg_run(const Op& A, uint32_t n, uint32_t len, co
     for (int q = 0; q < NC; ++q) {
       const uint32_t lc = threadIdx.x + q * T;
       if (lc < R.count) {
-        if (XS) xs[lc] = fma(alpha, p[lc], xs[lc]);
-        else P.x[R.c0 + lc] = fma(alpha, p[lc], P.x[R.c0 + lc]);
-        const double rn = fma(-alpha, z[q], r[lc]);
+        if (XS) xs[lc] = fma((V)alpha, p[lc], xs[lc]);
+        else P.x[R.c0 + lc] = fma((V)alpha, p[lc], P.x[R.c0 + lc]);
+        const V rn = fma(-(V)alpha, z[q], r[lc]);
         r[lc] = rn;
-        z[q] = (!PRE && P.inv ? P.inv[R.c0 + lc] : cells.inverse(A, q, R.c0 + lc)) * rn;
+        z[q] = rounded((!PRE && P.inv ? P.inv[R.c0 + lc] : cells.inverse(A, q, R.c0 + lc)) * rn);
         if (HALO) publish(lc, z[q]);
-        ab[0] += rn * rn;
-        ab[1] += rn * z[q];
+        ab[0] += (double)rn * (double)rn;
+        ab[1] += (double)rn * (double)z[q];
       }
     }
     if (!team.reduce(ab)) return;
-    const double res = sqrt(ab[0]);
+    double res = sqrt(ab[0]);
+    if (MIXED && isfinite(res) && (conv(res) || res <= P.delta * replaced || it == P.max_it)) {
+      flush_x();
+      if (!team.sync()) return;  // x of every block is in memory
+      if (!residual(ab)) return;
+      res = replaced = sqrt(ab[0]);
+      ++reps;
+      if (leader) *P.reps = (double)reps;
+    }
     if (leader && it < P.hist_cap) P.hist[it] = res;
     if (!isfinite(res)) return finish(CFDB_SOLVER_NONFINITE_RESIDUAL, it, res);
     res_cur = res;
@@ -683,7 +734,7 @@ __device__ __forceinline__ void spmv(const Op& A, const Cells<Op, NC ? NC : 1, (
   constexpr int G = NC ? NC : 2;
   const int sy = A.nx, sz = (int)A.sz;
   for (uint32_t g = threadIdx.x; g < R.count; g += G * T) {
-    Cf f[G];
+    Cf<double> f[G];
     double lo[G], hi[G];
 #pragma unroll
     for (int u = 0; u < G; ++u) {
@@ -770,7 +821,7 @@ __device__ __forceinline__ void bicgstab_run(const Op& A, uint32_t n, uint32_t l
   auto start = [&](double (&o)[1]) -> bool {
     o[0] = 0.0;
     each([&](int q, uint32_t lc, uint32_t c) {
-      const Cf f = cells.at(A, q, c);
+      const Cf<double> f = cells.at(A, q, c);
       const double rn = __ldg(P.b + c) - apply_global(A, f, c, P.x);
       r[lc] = rn;
       rh[lc] = rn;

@@ -1,6 +1,10 @@
-// The FP64 Jacobi-PCG of the p' operator with its vectors on chip
-// (resident.cuh): the systems that fit one thread-block cluster, or the
-// shared memory of the whole GPU.
+// The Jacobi-PCG of the p' operator with its vectors on chip (resident.cuh):
+// the systems that fit one thread-block cluster, or the shared memory of the
+// whole GPU.  FP64, mixed precision (FP32 directions) and FP32 (the inner
+// solves of the refinement form).  A mixed solve (us per iteration, streaming
+// kernel before): 128^2 3.8 (18.3), 64^3 10.6 (19.1), 96x80x64 14.5 (27.7),
+// 128^3 34.3 (43.2); a refinement's FP32 iteration: 130x128 4.8 (12.0),
+// 65x60x50 9.7 (24.3), 127x120x100 24.2 (61.9).
 #include <cuda_runtime.h>
 
 #include <type_traits>
@@ -13,32 +17,41 @@ namespace {
 
 using namespace res;
 
-template <int DIM, int NC>
+enum { FP64 = 0, MIXED = 1, FP32 = 2 };
+template <int KIND>
+using Value = typename std::conditional<KIND == FP32, float, double>::type;
+
+template <int DIM, int NC, int KIND>
 __global__ void __launch_bounds__(kClusterThreads, 1)
-    pcg_cluster(FaceOp<DIM> A, uint32_t n, uint32_t len, FastDiv dlen, Io P) {
-  extern __shared__ __align__(16) double sm[];
+    pcg_cluster(FaceOp<DIM, Value<KIND>> A, uint32_t n, uint32_t len, FastDiv dlen, IoT<Value<KIND>> P) {
+  extern __shared__ __align__(16) unsigned char sm[];
   __shared__ TeamSmem ts;
-  auto T = cluster_team<kClusterThreads>(&ts, len, dlen);
-  cg_run<kClusterThreads, NC, (NC <= 2), true, true>(A, n, len, P, T, sm);
+  auto team = cluster_team<kClusterThreads>(&ts, len, dlen);
+  cg_run<kClusterThreads, NC, (NC <= 2), true, true, KIND == MIXED>(
+      A, n, len, P, team, reinterpret_cast<Value<KIND>*>(sm));
 }
 
-template <int DIM, int T, int NC, bool XS, bool HALO>
+template <int DIM, int T, int NC, bool XS, bool HALO, int KIND>
 __global__ void __launch_bounds__(T, 1)
-    pcg_grid(FaceOp<DIM> A, uint32_t n, uint32_t len, GridWords w, Io P) {
-  extern __shared__ __align__(16) double sm[];
+    pcg_grid(FaceOp<DIM, Value<KIND>> A, uint32_t n, uint32_t len, GridWords w, IoT<Value<KIND>> P) {
+  extern __shared__ __align__(16) unsigned char sm[];
   __shared__ TeamSmem ts;
   auto team = grid_team<T>(&ts, w);
-  cg_run<T, NC, false, XS, HALO>(A, n, len, P, team, sm);
+  cg_run<T, NC, false, XS, HALO, KIND == MIXED>(A, n, len, P, team, reinterpret_cast<Value<KIND>*>(sm));
 }
 
 using ClusterNCs = std::integer_sequence<int, 1, 2, 3, 4, 6, 8>;
 using SmallNCs = std::integer_sequence<int, 1, 2, 4>;
 using LargeNCs = std::integer_sequence<int, 4, 8, 14>;
 
-template <int DIM>
-cfdb_status run(cfdb_context* ctx, const OpView<double>& V, const double* invd, const Plan& P,
-                uint32_t n, const Io& io) {
-  FaceOp<DIM> A{};
+template <int DIM, int KIND>
+cfdb_status run(cfdb_context* ctx, const OpView<Value<KIND>>& V, const Value<KIND>* invd,
+                const IoT<Value<KIND>>& io) {
+  const int64_t cells = (int64_t)V.nx * V.ny * V.nz;
+  const int limit = cluster_limit((const void*)pcg_cluster<DIM, 8, KIND>, kClusterThreads);
+  const Plan P = cg_plan(cells, (int64_t)V.nx * V.ny, ctx->num_sms, limit, sizeof(Value<KIND>));
+  const uint32_t n = (uint32_t)cells;
+  FaceOp<DIM, Value<KIND>> A{};
   A.A = V;
   A.invd = invd;
   A.nx = V.nx;
@@ -54,7 +67,7 @@ cfdb_status run(cfdb_context* ctx, const OpView<double>& V, const double* invd, 
   cudaError_t e;
   if (P.team == 1) {
     e = with_nc(P.nc, ClusterNCs{}, [&](auto nc) {
-      auto fn = pcg_cluster<DIM, decltype(nc)::value>;
+      auto fn = pcg_cluster<DIM, decltype(nc)::value, KIND>;
       if (cluster_limit((const void*)fn, kClusterThreads) < P.blocks) return cudaErrorInvalidConfiguration;
       return launch_cluster(fn, P.blocks, P.blocks, kClusterThreads, P.smem, ctx->stream, A, n, P.len,
                             fast_div(P.len), io);
@@ -62,15 +75,15 @@ cfdb_status run(cfdb_context* ctx, const OpView<double>& V, const double* invd, 
   } else {
     auto go = [&](auto threads, auto nc) {
       constexpr int T = decltype(threads)::value, NC = decltype(nc)::value;
-      const void* fn = P.halo ? (P.xs ? (const void*)pcg_grid<DIM, T, NC, true, true>
-                                      : (const void*)pcg_grid<DIM, T, NC, false, true>)
-                              : (P.xs ? (const void*)pcg_grid<DIM, T, NC, true, false>
-                                      : (const void*)pcg_grid<DIM, T, NC, false, false>);
+      const void* fn = P.halo ? (P.xs ? (const void*)pcg_grid<DIM, T, NC, true, true, KIND>
+                                      : (const void*)pcg_grid<DIM, T, NC, false, true, KIND>)
+                              : (P.xs ? (const void*)pcg_grid<DIM, T, NC, true, false, KIND>
+                                      : (const void*)pcg_grid<DIM, T, NC, false, false, KIND>);
       cudaError_t q = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMax);
       if (q != cudaSuccess) return q;
-      FaceOp<DIM> a = A;
+      auto a = A;
       uint32_t nn = n, len = P.len;
-      Io o = io;
+      auto o = io;
       void* args[] = {&a, &nn, &len, &w, &o};
       return cudaLaunchCooperativeKernel(fn, dim3(P.blocks), dim3(T), args, P.smem, ctx->stream);
     };
@@ -85,32 +98,41 @@ cfdb_status run(cfdb_context* ctx, const OpView<double>& V, const double* invd, 
   return CFDB_OK;
 }
 
-}  // namespace
-
-bool resident_pcg_fits(const cfdb_context* ctx, const OpView<double>& A) {
-  return cg_plan((int64_t)A.nx * A.ny * A.nz, (int64_t)A.nx * A.ny, ctx->num_sms, 0).team != 0;
-}
-
-cfdb_status resident_pcg(cfdb_context* ctx, const OpView<double>& A, int dim, const double* invd,
-                         const double* b, double* x, double* pub, double* inv,
-                         double abs_tol, double rel_tol,
-                         int64_t max_it, double* hist, int64_t hist_cap) {
-  const int64_t n = (int64_t)A.nx * A.ny * A.nz;
-  const int limit = dim == 2 ? cluster_limit((const void*)pcg_cluster<2, 8>, kClusterThreads)
-                             : cluster_limit((const void*)pcg_cluster<3, 8>, kClusterThreads);
-  const Plan P = cg_plan(n, (int64_t)A.nx * A.ny, ctx->num_sms, limit);
-  Io io{};
+template <typename V>
+IoT<V> io_of(cfdb_context* ctx, const V* b, V* x, V* pub, V* inv, const ResidentLimits& l) {
+  IoT<V> io{};
   io.b = b;
   io.x = x;
   io.pub = pub;
   io.inv = inv;
-  io.abs_tol = abs_tol;
-  io.rel_tol = rel_tol;
-  io.max_it = max_it;
-  io.hist = hist;
-  io.hist_cap = hist_cap;
+  io.abs_tol = l.abs_tol;
+  io.rel_tol = l.rel_tol;
+  io.max_it = l.max_it;
+  io.hist = l.hist;
+  io.hist_cap = l.hist_cap;
   io.out = ctx->scalars;
-  return dim == 2 ? run<2>(ctx, A, invd, P, (uint32_t)n, io) : run<3>(ctx, A, invd, P, (uint32_t)n, io);
+  io.delta = l.delta;
+  io.reps = ctx->scalars + l.reps_slot;
+  return io;
+}
+
+}  // namespace
+
+bool resident_pcg_fits(const cfdb_context* ctx, int nx, int ny, int nz, size_t word) {
+  return cg_plan((int64_t)nx * ny * nz, (int64_t)nx * ny, ctx->num_sms, 0, word).team != 0;
+}
+
+cfdb_status resident_pcg(cfdb_context* ctx, const OpView<double>& A, int dim, const double* invd,
+                         const double* b, double* x, double* pub, double* inv, const ResidentLimits& l) {
+  const auto io = io_of<double>(ctx, b, x, pub, inv, l);
+  if (l.delta > 0.0) return dim == 2 ? run<2, MIXED>(ctx, A, invd, io) : run<3, MIXED>(ctx, A, invd, io);
+  return dim == 2 ? run<2, FP64>(ctx, A, invd, io) : run<3, FP64>(ctx, A, invd, io);
+}
+
+cfdb_status resident_pcg(cfdb_context* ctx, const OpView<float>& A, int dim, const float* invd,
+                         const float* b, float* x, float* pub, float* inv, const ResidentLimits& l) {
+  const auto io = io_of<float>(ctx, b, x, pub, inv, l);
+  return dim == 2 ? run<2, FP32>(ctx, A, invd, io) : run<3, FP32>(ctx, A, invd, io);
 }
 
 }  // namespace cfdb

@@ -48,7 +48,7 @@ constexpr int64_t kClusterCells = 36864;
 // 40x33 2.7 (18.6), 129^2 4.7 (13.0), 512^2 8.0 (20.9), 64^3 9.6 (19.5),
 // 96^3 16.7 (29.3), 128^3 31.8 (44.7); the last two keep no neighbouring
 // planes.  `reach`: cells the stencil reaches (a plane).
-inline Plan cg_plan(int64_t n, int64_t reach, int num_sms, int max_cluster) {
+inline Plan cg_plan(int64_t n, int64_t reach, int num_sms, int max_cluster, size_t word = 8) {
   Plan P;
   auto fill = [&](int team, int blocks, int max_nc, bool halo) {
     P = Plan{};
@@ -60,8 +60,8 @@ inline Plan cg_plan(int64_t n, int64_t reach, int num_sms, int max_cluster) {
     P.nc = (int)((P.len + threads - 1) / threads);
     P.halo = halo;
     const size_t words = (size_t)P.len * (team == 1 ? 3 : 2) + (halo ? 2 * (size_t)reach : 0);
-    P.xs = (words + P.len) * 8 <= kSmemMax;
-    P.smem = (words + (P.xs ? P.len : 0)) * 8;
+    P.xs = (words + P.len) * word <= kSmemMax;
+    P.smem = (words + (P.xs ? P.len : 0)) * word;
     // a cluster's kernel has x in shared memory always
     if (P.nc <= max_nc && P.smem <= kSmemMax && (team == 2 || P.xs)) P.team = team;
   };
