@@ -742,7 +742,7 @@ __device__ __forceinline__ void coarse_fetch_levels(const CoarsePlan& P, float* 
 // a named barrier of its own (the others wait where they are needed again),
 // the scaled residual u is formed where r is, and prolongation and Jacobi
 // sweeps need no phase of their own (x + c P e is formed as it is read, the
-// sweeps alternate between two vectors).  With it a 24^3 FCG iteration takes
+// sweeps alternate between two vectors).  With it a 24^3 FCG iteration took
 // 37 us instead of 41, 12^3 21 instead of 26.
 template <int DIM>
 __device__ __forceinline__ void coarse_cycle(const CoarsePlan& P, float* sm) {
@@ -1069,8 +1069,8 @@ size_t coarse_bytes(const MgHierarchy& H, int from) {
   return floats * sizeof(float);
 }
 
-// The levels [from, ...) in one block.
-CoarsePlan coarse_plan(const MgHierarchy& H, const MgWeights& W, int from) {
+// The levels [from, ...) in one block of `threads`.
+CoarsePlan coarse_plan(const MgHierarchy& H, const MgWeights& W, int from, int threads) {
   CoarsePlan P;
   std::memset(&P, 0, sizeof(P));
   P.count = H.levels - from;
@@ -1100,7 +1100,7 @@ CoarsePlan coarse_plan(const MgHierarchy& H, const MgWeights& W, int from) {
     c.off[6] = take(coarse_padded(H.dim, c.n));        // u (padded)
     c.dx = res::fast_div(c.n[0]);
     c.dy = res::fast_div(c.n[1]);
-    c.warps = std::min(kCoarseThreads / 32, (c.cells + 31) / 32);
+    c.warps = std::min(threads / 32, (c.cells + 31) / 32);
     P.K[q] = kern_of(W, from + q);
     P.cw[q] = cw_of(W, from + q);
   }
@@ -1407,9 +1407,9 @@ void level_sm(const MgLevel& M, const LV& LC, const Kern& K, bool first, const f
 // (257), 80x48x48 96.0 (101), 100x75x61 134 (142), 256^3 752 (754).
 constexpr int64_t kTailCells = 32768;
 // Systems of at most this many cells run their whole FCG loop in a cluster
-// where it has the shared memory (2D to 256^2, 3D to about 36^3): 129^2 29.6
-// us an iteration (graph of grid kernels: 55.8), 256^2 42 (57.6), 12^3 21
-// (48), 24^3 37 (62), 33^3 56 (76).
+// where it has the shared memory (2D to 256^2, 3D to about 36^3): 129^2 26.6
+// us an iteration (graph of grid kernels: 55.8), 256^2 40 (57.6), 12^3 14
+// (48), 24^3 29 (62), 33^3 48 (76).
 constexpr int64_t kFcgClusterCells = 65536;
 
 // Whether `fn` can run as a cluster of kMaxCluster blocks.
@@ -1478,7 +1478,7 @@ int enqueue_cycle(const MgHierarchy& H, const MgWeights& W, const float* r0, flo
     launch_in_cluster(k_tail<DIM>, sizeof(float) * (size_t)CL.words, st, CL.P, CL.Q, CL.words);
     ++launches;
   } else if (cf < H.levels) {
-    const CoarsePlan P = coarse_plan(H, W, cf);
+    const CoarsePlan P = coarse_plan(H, W, cf, kCoarseThreads);
     launch(k_coarse<DIM>, 1, kCoarseThreads, H.coarse_smem + sizeof(float) * plan_words<CoarsePlan>(), st, P);
     ++launches;
   }

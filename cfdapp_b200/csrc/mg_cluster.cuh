@@ -5,22 +5,22 @@
 // its own it takes 3.5-4 us, and inside one kernel with its vectors in L2 and
 // a cluster barrier between passes still 2 us (a trip to L2 for the loads and
 // one for the stores before the barrier).  Here the vectors of the small
-// levels live in the shared memory of a cluster of 16 blocks of 1024 threads.
+// levels live in the shared memory of a cluster of 16 blocks of 512 threads
+// (with 1024 the barriers and sums cost more than the passes gain: an FCG
+// iteration of 24^2 14.3 against 10.4 us, 129^2 29.5 / 26.6, 24^3 36.9 / 28.9).
 // Every block owns a run of planes of each level (z in kernel space), aligned
 // so that a coarse plane's children belong to its owner; each vector that a
 // stencil reads keeps one halo plane per side, which the neighbours push into
 // it through distributed shared memory as they compute; a hardware cluster
 // barrier ends each pass.  Couplings and scales come through L1.  The
 // coarsest levels run in the first block (coarse_cycle).  What bounds it now
-// is instruction issue and the chain of passes on 16 SMs: at 129^2 a pass of
-// the finest level takes 1.2-2.5 us, the block-resident levels 9 us of a
-// 30 us iteration.
+// is instruction issue and the chain of passes on 16 SMs.
 //
 //   k_tail         the levels below the grid kernels' in one launch
 //   k_fcg_cluster  the whole FCG loop of a small system: one launch a solve
 #pragma once
 
-constexpr int kClusterT = 1024;
+constexpr int kClusterT = 512;
 constexpr int kMaxTail = 6;
 
 using ClusterT = res::ClusterTeam<kClusterT>;
@@ -554,7 +554,7 @@ ClusterLayout cluster_layout(const MgHierarchy& H, const MgWeights& W, int from,
     if ((off + own) * 4 <= (int64_t)res::kSmemMax) P.ox64 = take(own);
   }
   if ((size_t)off * 4 > res::kSmemMax) return C;
-  C.Q = coarse_plan(H, W, cf);
+  C.Q = coarse_plan(H, W, cf, kClusterT);
   C.words = off;
   return C;
 }
