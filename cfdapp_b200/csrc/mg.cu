@@ -417,7 +417,7 @@ constexpr int kRunning = -1;
 
 // Block partials -> fixed-order total in the last block; fin(tot) runs in
 // thread 0 of that block.  Every thread of the block must call this.
-template <int NV, class Fin>
+template <int NV, bool WIDE = true, class Fin>
 __device__ __forceinline__ void reduce_last(double (&v)[NV], double* partials, unsigned* ticket,
                                             Fin fin) {
   __shared__ double red[32 * NV];
@@ -435,7 +435,21 @@ __device__ __forceinline__ void reduce_last(double (&v)[NV], double* partials, u
   if (is_last) {
     __threadfence();
     double tot[NV];
-    grid_total<NV>(partials, NV, nb, tot, red);
+    if constexpr (WIDE) {
+      // every thread of the block takes a strided share of the partials: one
+      // warp alone spends several trips to L2 on the 1 000-2 400 of a wide
+      // pass (an FCG iteration of 100x75x61 134 -> 128 us; blocks of 64
+      // threads gain nothing)
+#pragma unroll
+      for (int q = 0; q < NV; ++q) tot[q] = 0.0;
+#pragma unroll 4
+      for (int p = threadIdx.x; p < nb; p += blockDim.x)
+#pragma unroll
+        for (int q = 0; q < NV; ++q) tot[q] += __ldcg(partials + (size_t)p * NV + q);
+      block_sum<NV>(tot, red);
+    } else {
+      grid_total<NV>(partials, NV, nb, tot, red);
+    }
     if (threadIdx.x == 0) {
       fin(tot);
       atomicExch(ticket, 0u);

@@ -339,7 +339,7 @@ __global__ void __launch_bounds__(Quad<DIM>::TX* Quad<DIM>::TY)
   });
   if (HOOK) {
     double acc[1] = {acc_dot};
-    reduce_last<1>(acc, hk.partials, &hk.S->ticket, [&](const double* tot) {
+    reduce_last<1, DIM == 3>(acc, hk.partials, &hk.S->ticket, [&](const double* tot) {
       FcgState* S = hk.S;
       if (S->it == 0) return;  // the first direction is z itself
       const double beta = tot[0] / S->pq;
@@ -457,7 +457,7 @@ __global__ void __launch_bounds__(Quad<DIM>::TX* Quad<DIM>::TY, dir_blocks_per_s
         },
         [](int) {});
   });
-  reduce_last<2>(acc, partials, &S->ticket, [&](const double* tot) {
+  reduce_last<2, DIM == 3>(acc, partials, &S->ticket, [&](const double* tot) {
     const double pq = tot[0], pr = tot[1];
     const double alpha = pr / pq;
     if (!isfinite(pq) || !(pq > 0.0) || !isfinite(alpha)) {
