@@ -5,19 +5,12 @@
 // follows).
 //
 // Work layout.  Everything runs in kernel space (2D grids as nx x 1 x ny).
-// Fine levels use plane-marching tiles: a 256-thread block owns a 32x8 (3D)
-// or 256x1 (2D) patch of an (x,y) plane and marches along z through a run of
-// planes, staging each plane with a one-cell halo in shared memory, so every
-// array is read from DRAM about once per pass and neighbours come from
-// shared memory.  Residual passes use the 7-point cross (z-neighbours kept in
-// registers); smoothing passes use the 27-point (9-point in 2D) convolution
-// over a three-plane ring.  The restriction to the next level is fused into
-// the last residual pass of a level: plane runs start on even planes, so the
-// 2x2x2 children of a coarse cell are summed inside one block (shuffle in x,
-// shared memory in y, a register across the z pair) -- deterministic, no
-// atomics.  All levels at or below 4096 cells run inside ONE thread block
-// with their data in shared memory; the levels above them up to 32768 cells,
-// and the whole solve of a small system, on one cluster (mg_cluster.cuh).
+// Large levels with rows of whole tiles march in z with four cells per thread
+// (mg_quad.cuh), so every array is read from DRAM about once per pass; other
+// levels gather, one cell per thread (mg_gather.cuh).  All levels at or below
+// 4096 cells run inside ONE thread block with their data in shared memory;
+// the levels above them up to 32768 cells, and the whole solve of a small
+// system, on one cluster (mg_cluster.cuh).
 //
 // Reductions are deterministic without a grid barrier: every block stores its
 // partial sums, and the last block to finish (atomic ticket) adds all partials
@@ -255,7 +248,6 @@ int seg_grid(const Seg& s) {
   return (int)std::max<int64_t>(1, (s.items + per - 1) / per);
 }
 
-// Four cells per thread where the level is wide enough.
 // f(tix, tiy, k0, k1) for every plane run of this block.
 template <class F>
 __device__ __forceinline__ void for_runs(const Seg& sg, int nz, F f) {
@@ -336,65 +328,6 @@ __device__ __forceinline__ void march7(int nx, int ny, int nz, int tix, int tiy,
     }
   }
   __syncthreads();
-}
-
-// 27-point (2D: 9-point) convolution march over a three-plane ring: u(i,j,k)
-// is the convolved field; cell(c, act, i, j, k, sum) runs for each of the
-// thread's CX cells of every plane with sum = sum_o K[o] u(cell+o) (0 outside
-// the domain).
-template <int TX, int TY, int CX, bool TWO_D, class U, class Cell>
-__device__ __forceinline__ void march27(int nx, int ny, int nz, int tix, int tiy, int k0, int k1,
-                                        float (*ring)[Rows<TY>::N][TX * CX + 2], const Kern& K,
-                                        U u, Cell cell) {
-  constexpr int PX = TX * CX, R0 = Rows<TY>::R0;
-  static_assert(!TWO_D || TY == 1, "a 2D plane is one row");
-  const int tid = threadIdx.x;
-  const int tx = tid % TX, ty = tid / TX;
-  const int x0 = tix * PX, j = tiy * TY + ty;
-  auto load = [&](int kp, int slot) {
-    float(*s)[PX + 2] = ring[slot];
-    const bool zin = kp >= 0 && kp < nz;
-    if (TWO_D) {
-      for (int q = tid; q < PX + 2; q += TX * TY) {
-        const int gi = x0 + q - 1;
-        s[0][q] = (zin && gi >= 0 && gi < nx) ? u(gi, 0, kp) : 0.f;
-      }
-    } else {
-      for (int q = tid; q < (TY + 2) * (PX + 2); q += TX * TY) {
-        const int hy = q / (PX + 2), hx = q % (PX + 2);
-        const int gi = x0 + hx - 1, gj = tiy * TY + hy - 1;
-        s[hy][hx] = (zin && gi >= 0 && gi < nx && gj >= 0 && gj < ny) ? u(gi, gj, kp) : 0.f;
-      }
-    }
-  };
-  // slots rotate: lo holds plane k-1, mi plane k, hi plane k+1
-  int lo = 0, mi = 1, hi = 2;
-  load(k0 - 1, lo);
-  load(k0, mi);
-  for (int k = k0; k < k1; ++k) {
-    load(k + 1, hi);
-    __syncthreads();
-    const float(*pl[3])[PX + 2] = {ring[lo], ring[mi], ring[hi]};  // planes k-1, k, k+1
-#pragma unroll
-    for (int c = 0; c < CX; ++c) {
-      const int xi = 1 + tx + c * TX;
-      float sum = 0.f;
-#pragma unroll
-      for (int dk = 0; dk < 3; ++dk)
-#pragma unroll
-        for (int dj = (TWO_D ? 0 : -1); dj <= (TWO_D ? 0 : 1); ++dj)
-#pragma unroll
-          for (int di = -1; di <= 1; ++di)
-            sum += K.w[dk * 9 + (dj + 1) * 3 + (di + 1)] * pl[dk][ty + R0 + dj][xi + di];
-      const int i = x0 + tx + c * TX;
-      cell(c, j < ny && i < nx, i, j, k, sum);
-    }
-    __syncthreads();
-    const int t = lo;
-    lo = mi;
-    mi = hi;
-    hi = t;
-  }
 }
 
 // ----------------------------------------------------------------- FCG state
@@ -483,67 +416,6 @@ struct Hook {
 
 // ------------------------------------------------------------ level kernels
 
-// res = r - A x  (PRO: x + cw P ec in place of x).  RESTRICT: instead of
-// storing res, rc(parent) = sum of the children's res.  r[skip] reads as 0.
-template <int DIM, int CX, bool PRO, bool RESTRICT>
-__global__ void __launch_bounds__(kT) k_res(LV L, LV C, Seg sg, const float* __restrict__ x,
-                                            const float* __restrict__ ec, float cw,
-                                            const float* __restrict__ r, float* __restrict__ res,
-                                            float* __restrict__ rc, int64_t skip) {
-  pdl_enter();
-  constexpr int TX = Tile<DIM>::TX, TY = Tile<DIM>::TY, PX = TX * CX;
-  __shared__ float buf[2][Rows<TY>::N][PX + 2];
-  __shared__ float rows[TY][CX][TX / 2];
-  const int tx = threadIdx.x % TX, ty = threadIdx.x / TX;
-  auto val = [&](int i, int j, int k) {
-    float v = x[at(L, i, j, k)];
-    if (PRO) v += cw * ec[parent(C, i, j, k)];
-    return v;
-  };
-  for_runs(sg, L.nz, [&](int tix, int tiy, int k0, int k1) {
-    float rv[CX], racc[CX];
-#pragma unroll
-    for (int c = 0; c < CX; ++c) racc[c] = 0.f;
-    const int x0 = tix * PX, j = tiy * TY + ty;
-    march7<float, TX, TY, CX>(
-        L.nx, L.ny, L.nz, tix, tiy, k0, k1, buf, val,
-        [&](int c, bool act, int i, int jj, int k, float v, float w, float e, float s, float n,
-            float b, float t) {
-          rv[c] = 0.f;
-          if (act) {
-            const int64_t q = at(L, i, jj, k);
-            rv[c] = (q == skip ? 0.f : r[q]) - apply7(coef<DIM>(L, i, jj, k), v, w, e, s, n, b, t);
-            if (!RESTRICT) res[q] = rv[c];
-          }
-        },
-        [&](int k) {
-          if constexpr (!RESTRICT) return;
-          float quad[CX];
-#pragma unroll
-          for (int c = 0; c < CX; ++c) quad[c] = rv[c] + __shfl_xor_sync(0xffffffffu, rv[c], 1);
-          if (TY > 1) {
-            if ((tx & 1) == 0)
-#pragma unroll
-              for (int c = 0; c < CX; ++c) rows[ty][c][tx >> 1] = quad[c];
-            __syncthreads();
-            if ((tx & 1) == 0 && (ty & 1) == 0)
-#pragma unroll
-              for (int c = 0; c < CX; ++c) quad[c] += rows[ty + 1][c][tx >> 1];
-          }
-          const bool writer = (tx & 1) == 0 && (TY == 1 || (ty & 1) == 0);
-          const bool flush = (k & 1) == 1 || k + 1 == L.nz;
-#pragma unroll
-          for (int c = 0; c < CX; ++c) {
-            racc[c] = ((k & 1) == 0) ? quad[c] : racc[c] + quad[c];
-            if (writer && flush) {
-              const int ci = (x0 + tx + c * TX) >> 1, cj = j >> 1, ck = k >> 1;
-              if (ci < C.nx && cj < C.ny) rc[ci + (int64_t)C.nx * (cj + (int64_t)C.ny * ck)] = racc[c];
-            }
-          }
-        });
-  });
-}
-
 enum { SM_FIRST = 0, SM_ADD = 1 };
 
 #ifndef CFDB_PDL
@@ -576,50 +448,6 @@ void launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaSt
   cfg.numAttrs = 1;
   const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
   if (e != cudaSuccess && g_launch_error == cudaSuccess) g_launch_error = e;
-}
-
-// x <- [x] (+ cw P ec) + D^-1/2 (W * (D^-1/2 u)), u = res (SM_ADD) or r with
-// r[skip] = 0 and x = 0 before (SM_FIRST).  pin >= 0: z[pin] = r[pin] (the
-// last sweep of level 0); HOOK: also accumulate z.q for the FCG coefficient.
-template <int DIM, int CX, int MODE, bool HOOK>
-__global__ void __launch_bounds__(kT) k_sm(LV L, LV C, Seg sg, Kern K, const float* __restrict__ src,
-                                           const float* __restrict__ ec, float cw,
-                                           float* __restrict__ x, int64_t skip, int64_t pin,
-                                           const float* __restrict__ r, Hook hk) {
-  pdl_enter();
-  constexpr int TX = Tile<DIM>::TX, TY = Tile<DIM>::TY, PX = TX * CX;
-  __shared__ float ring[3][Rows<TY>::N][PX + 2];
-  double acc[1] = {0.0};
-  auto u = [&](int i, int j, int k) {
-    const int64_t q = at(L, i, j, k);
-    if (MODE == SM_FIRST && q == skip) return 0.f;
-    return src[q] * L.isq[q];
-  };
-  for_runs(sg, L.nz, [&](int tix, int tiy, int k0, int k1) {
-    march27<TX, TY, CX, DIM == 2>(L.nx, L.ny, L.nz, tix, tiy, k0, k1, ring, K, u,
-                                  [&](int, bool act, int i, int j, int k, float sum) {
-                                    if (!act) return;
-                                    const int64_t c = at(L, i, j, k);
-                                    float v = L.isq[c] * sum;
-                                    if (MODE == SM_ADD) v += x[c];
-                                    if (ec) v += cw * ec[parent(C, i, j, k)];
-                                    if (c == pin) v = r[c];
-                                    x[c] = v;
-                                    if (HOOK) acc[0] += (double)v * hk.q[c];
-                                  });
-  });
-  if (HOOK) {
-    reduce_last<1>(acc, hk.partials, &hk.S->ticket, [&](const double* tot) {
-      FcgState* S = hk.S;
-      if (S->it == 0) return;  // the first direction is z itself
-      const double beta = tot[0] / S->pq;
-      if (!isfinite(beta)) {
-        stop_loop(S, hk.h, kLearnedStagnated);
-        return;
-      }
-      S->beta = beta;
-    });
-  }
 }
 
 // ----------------------------------------------------- coarse-level block
@@ -1121,154 +949,18 @@ CoarsePlan coarse_plan(const MgHierarchy& H, const MgWeights& W, int from, int t
   return P;
 }
 
-// -------------------------------------------------- flat small-level passes
-//
-// Levels of at most kFlatCells cells are latency-bound: a plane march would
-// chain a few dependent load/barrier steps per block for almost no data.
-// These passes give every cell its own thread (all loads independent), so a
-// pass costs about one memory latency.
-constexpr int64_t kFlatCells = 1 << 16;
-
-__device__ __forceinline__ void cell_ijk(const LV& L, int64_t c, int& i, int& j, int& k) {
-  i = (int)(c % L.nx);
-  const int64_t rest = c / L.nx;
-  j = (int)(rest % L.ny);
-  k = (int)(rest / L.ny);
-}
-
-// res = r - A x (PRO: x + cw P ec in place of x), r[skip] read as 0
-template <int DIM, bool PRO>
-__global__ void __launch_bounds__(256) k_res_f(LV L, LV C, const float* __restrict__ x,
-                                               const float* __restrict__ ec, float cw,
-                                               const float* __restrict__ r, float* __restrict__ res,
-                                               int64_t skip) {
-  pdl_enter();
-  const int64_t n = (int64_t)L.nx * L.ny * L.nz;
-  for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < n;
-       c += (int64_t)gridDim.x * blockDim.x) {
-    int i, j, k;
-    cell_ijk(L, c, i, j, k);
-    const int64_t plane = (int64_t)L.nx * L.ny;
-    auto xv = [&](int64_t q, int ii, int jj, int kk) {
-      float v = x[q];
-      if (PRO) v += cw * ec[parent(C, ii, jj, kk)];
-      return v;
-    };
-    const float v = xv(c, i, j, k);
-    const float w = i > 0 ? xv(c - 1, i - 1, j, k) : 0.f;
-    const float e = i + 1 < L.nx ? xv(c + 1, i + 1, j, k) : 0.f;
-    const float s = (DIM == 3 && j > 0) ? xv(c - L.nx, i, j - 1, k) : 0.f;
-    const float nn = (DIM == 3 && j + 1 < L.ny) ? xv(c + L.nx, i, j + 1, k) : 0.f;
-    const float b = k > 0 ? xv(c - plane, i, j, k - 1) : 0.f;
-    const float t = k + 1 < L.nz ? xv(c + plane, i, j, k + 1) : 0.f;
-    res[c] = (c == skip ? 0.f : r[c]) - apply7(coef<DIM>(L, i, j, k), v, w, e, s, nn, b, t);
-  }
-}
-
-// rc(C) = sum of the children's (r - A x)
-template <int DIM>
-__global__ void __launch_bounds__(256) k_restrict_f(LV L, LV C, const float* __restrict__ x,
-                                                    const float* __restrict__ r,
-                                                    float* __restrict__ rc, int64_t skip) {
-  pdl_enter();
-  const int64_t n = (int64_t)C.nx * C.ny * C.nz;
-  for (int64_t qc = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; qc < n;
-       qc += (int64_t)gridDim.x * blockDim.x) {
-    int ci, cj, ck;
-    cell_ijk(C, qc, ci, cj, ck);
-    float sum = 0.f;
-    for (int u = 0; u < 2; ++u)
-      for (int v = 0; v < 2; ++v)
-        for (int t = 0; t < 2; ++t) {
-          const int i = 2 * ci + t, j = 2 * cj + v, k = 2 * ck + u;
-          if (i >= L.nx || j >= L.ny || k >= L.nz) continue;
-          const int64_t c = at(L, i, j, k);
-          const int64_t plane = (int64_t)L.nx * L.ny;
-          const float w = i > 0 ? x[c - 1] : 0.f, e = i + 1 < L.nx ? x[c + 1] : 0.f;
-          const float s = (DIM == 3 && j > 0) ? x[c - L.nx] : 0.f;
-          const float nn = (DIM == 3 && j + 1 < L.ny) ? x[c + L.nx] : 0.f;
-          const float b = k > 0 ? x[c - plane] : 0.f, tt = k + 1 < L.nz ? x[c + plane] : 0.f;
-          sum += (c == skip ? 0.f : r[c]) - apply7(coef<DIM>(L, i, j, k), x[c], w, e, s, nn, b, tt);
-        }
-    rc[qc] = sum;
-  }
-}
-
-// x <- [x] (+ cw P ec) + D^-1/2 (W * (D^-1/2 u)), u = res, or r (r[skip]
-// = 0) from x = 0 (FIRST); pin >= 0: x[pin] = r[pin]
-template <int DIM, int MODE>
-__global__ void __launch_bounds__(256) k_sm_f(LV L, LV C, Kern K, const float* __restrict__ src,
-                                              const float* __restrict__ ec, float cw,
-                                              float* __restrict__ x, int64_t skip, int64_t pin,
-                                              const float* __restrict__ r) {
-  pdl_enter();
-  const int64_t n = (int64_t)L.nx * L.ny * L.nz;
-  for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < n;
-       c += (int64_t)gridDim.x * blockDim.x) {
-    int i, j, k;
-    cell_ijk(L, c, i, j, k);
-    float sum = 0.f;
-#pragma unroll
-    for (int dk = -1; dk <= 1; ++dk) {
-      const int kk = k + dk;
-      if (kk < 0 || kk >= L.nz) continue;
-#pragma unroll
-      for (int dj = (DIM == 2 ? 0 : -1); dj <= (DIM == 2 ? 0 : 1); ++dj) {
-        const int jj = j + dj;
-        if (jj < 0 || jj >= L.ny) continue;
-#pragma unroll
-        for (int di = -1; di <= 1; ++di) {
-          const int ii = i + di;
-          if (ii < 0 || ii >= L.nx) continue;
-          const int64_t q = at(L, ii, jj, kk);
-          const float u = (MODE == SM_FIRST && q == skip) ? 0.f : src[q] * L.isq[q];
-          sum += K.w[(dk + 1) * 9 + (dj + 1) * 3 + (di + 1)] * u;
-        }
-      }
-    }
-    float v = L.isq[c] * sum;
-    if (MODE == SM_ADD) v += x[c];
-    if (ec) v += cw * ec[parent(C, i, j, k)];
-    if (c == pin) v = r[c];
-    x[c] = v;
-  }
-}
-
-int flat_blocks(int64_t n) {
-  return (int)std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, 148 * 8));
-}
+// Levels of at most this many cells gather even where the quad kernels could
+// take them: a march chains a few dependent load and barrier steps per block
+// for almost no data.  FCG iteration (us) with 2^16 / 2^19 / 2^21: 512^2
+// 70.0 / 65.7 / 63.5, 1024^2 120 / 112.8 / 117.4, 2048^2 242 / 232.5 / 236,
+// 128x100x90 - / 155 / 166, 128^3 199 / 199 / 247.
+constexpr int64_t kGatherCells = 1 << 19;
+// The 2D direction pass likewise: 300^2 57.0 -> 54.0 us, 512^2 63.5 -> 66.2.
+constexpr int64_t kGatherDirCells = 1 << 17;
 
 #include "mg_quad.cuh"
 #include "mg_stage.cuh"
-
-// Launchers of one level's passes, with the cells-per-thread choice.
-template <int DIM, int CX>
-struct LevelOps {
-  static void res(const MgLevel& M, const LV& LC, const float* x, const float* ec, float cw,
-                  const float* r, float* res, float* rc, int64_t skip, cudaStream_t st) {
-    const Seg sg = make_seg<DIM, CX>(M.n[0], M.n[1], M.n[2]);
-    const LV L = lv(M);
-    if (rc)
-      launch(k_res<DIM, CX, false, true>, seg_grid(sg), kT, 0, st, L, LC, sg, x, ec, cw, r, res, rc, skip);
-    else if (ec)
-      launch(k_res<DIM, CX, true, false>, seg_grid(sg), kT, 0, st, L, LC, sg, x, ec, cw, r, res, rc, skip);
-    else
-      launch(k_res<DIM, CX, false, false>, seg_grid(sg), kT, 0, st, L, LC, sg, x, ec, cw, r, res, rc, skip);
-  }
-  static void sm(const MgLevel& M, const LV& LC, const Kern& K, bool first, const float* src,
-                 const float* ec, float cw, float* x, int64_t skip, int64_t pin, const float* r,
-                 const Hook* hook, cudaStream_t st) {
-    const Seg sg = make_seg<DIM, CX>(M.n[0], M.n[1], M.n[2]);
-    const LV L = lv(M);
-    const int g = seg_grid(sg);
-    if (first)
-      launch(k_sm<DIM, CX, SM_FIRST, false>, g, kT, 0, st, L, LC, sg, K, src, ec, cw, x, skip, pin, r, Hook{});
-    else if (hook)
-      launch(k_sm<DIM, CX, SM_ADD, true>, g, kT, 0, st, L, LC, sg, K, src, ec, cw, x, skip, pin, r, *hook);
-    else
-      launch(k_sm<DIM, CX, SM_ADD, false>, g, kT, 0, st, L, LC, sg, K, src, ec, cw, x, skip, pin, r, Hook{});
-  }
-};
+#include "mg_gather.cuh"
 
 // Blocks of `fn` resident on the whole current GPU at `threads` threads per
 // block and `dyn` bytes of dynamic shared memory (registers and shared
@@ -1326,18 +1018,34 @@ void warm_quad_waves() {
   quad_wave<3>((const void*)k_dir_s<false>, sg, dir_s_smem());
 }
 
+// Whether a level's passes gather (mg_gather.cuh) rather than march in quads.
+// Their residual passes leave u = D^-1/2 res for their smoothing passes.
+template <int DIM>
+bool gathers(const MgLevel& M) {
+  return !quad_ok<DIM>(M.n[0]) || M.cells <= kGatherCells;
+}
+GLevel gcoarse(const LV& C) {
+  GLevel G;
+  G.L = C;
+  G.dx = res::fast_div(C.nx);
+  G.dy = res::fast_div(C.ny);
+  G.n = C.nx * C.ny * C.nz;
+  return G;
+}
+
 template <int DIM>
 void level_res(const MgLevel& M, const LV& LC, const float* x, const float* ec, float cw,
                const float* r, float* res, float* rc, int64_t skip, cudaStream_t st) {
-  if (M.cells <= kFlatCells) {
-    const LV L = lv(M);
+  if (gathers<DIM>(M)) {
+    const GLevel G = glevel(M);
+    const int g = gather_blocks(M.cells);
     if (rc) {
-      const int64_t nc = (int64_t)LC.nx * LC.ny * LC.nz;
-      launch(k_restrict_f<DIM>, flat_blocks(nc), 256, 0, st, L, LC, x, r, rc, skip);
+      const GLevel C = gcoarse(LC);
+      launch(k_restrict_g<DIM>, gather_blocks(C.n), 256, 0, st, G, C, x, r, rc, (int)skip);
     } else if (ec) {
-      launch(k_res_f<DIM, true>, flat_blocks(M.cells), 256, 0, st, L, LC, x, ec, cw, r, res, skip);
+      launch(k_resid_g<DIM, true>, g, 256, 0, st, G, LC, x, ec, cw, r, res, (int)skip);
     } else {
-      launch(k_res_f<DIM, false>, flat_blocks(M.cells), 256, 0, st, L, LC, x, ec, cw, r, res, skip);
+      launch(k_resid_g<DIM, false>, g, 256, 0, st, G, LC, x, ec, cw, r, res, (int)skip);
     }
   } else if (DIM == 3 && quad_ok<DIM>(M.n[0])) {
     const Seg sg = make_quad_seg<3>(M.n[0], M.n[1], M.n[2]);
@@ -1353,7 +1061,7 @@ void level_res(const MgLevel& M, const LV& LC, const float* x, const float* ec, 
     else
       launch(k_res_s<false, false>, quad_wave<3>((const void*)k_res_s<false, false>, sg, SM), T, SM,
              st, L, LC, sg, x, ec, cw, r, res, rc, skip);
-  } else if (quad_ok<DIM>(M.n[0])) {
+  } else {
     const Seg sg = make_quad_seg<DIM>(M.n[0], M.n[1], M.n[2]);
     constexpr int T = Quad<DIM>::TX * Quad<DIM>::TY;
     const LV L = lv(M);
@@ -1366,8 +1074,6 @@ void level_res(const MgLevel& M, const LV& LC, const float* x, const float* ec, 
     else
       launch(k_res_q<DIM, false, false>, quad_wave<DIM>((const void*)k_res_q<DIM, false, false>, sg), T,
              0, st, L, LC, sg, x, ec, cw, r, res, rc, skip);
-  } else {
-    LevelOps<DIM, 1>::res(M, LC, x, ec, cw, r, res, rc, skip, st);
   }
 }
 
@@ -1375,12 +1081,15 @@ template <int DIM>
 void level_sm(const MgLevel& M, const LV& LC, const Kern& K, bool first, const float* src,
               const float* ec, float cw, float* x, int64_t skip, int64_t pin, const float* r,
               const Hook* hook, cudaStream_t st) {
-  if (M.cells <= kFlatCells && !hook) {
-    const LV L = lv(M);
+  if (gathers<DIM>(M)) {
+    const GLevel G = glevel(M);
+    const int g = gather_blocks(M.cells);
     if (first)
-      launch(k_sm_f<DIM, SM_FIRST>, flat_blocks(M.cells), 256, 0, st, L, LC, K, src, ec, cw, x, skip, pin, r);
+      launch(k_first_g<DIM>, g, 256, 0, st, G, K, src, x, (int)skip);
+    else if (hook)
+      launch(k_smooth_g<DIM, true>, g, 256, 0, st, G, LC, K, src, ec, cw, x, (int)pin, r, *hook);
     else
-      launch(k_sm_f<DIM, SM_ADD>, flat_blocks(M.cells), 256, 0, st, L, LC, K, src, ec, cw, x, skip, pin, r);
+      launch(k_smooth_g<DIM, false>, g, 256, 0, st, G, LC, K, src, ec, cw, x, (int)pin, r, Hook{});
   } else if (DIM == 3 && quad_ok<DIM>(M.n[0])) {
     const Seg sg = make_quad_seg<3>(M.n[0], M.n[1], M.n[2]);
     constexpr int T = PlaneTile::T;
@@ -1395,7 +1104,7 @@ void level_sm(const MgLevel& M, const LV& LC, const Kern& K, bool first, const f
     else
       launch(k_sm_s<SM_ADD, false>, quad_wave<3>((const void*)k_sm_s<SM_ADD, false>, sg, SM), T, SM,
              st, L, LC, sg, K, src, ec, cw, x, skip, pin, r, Hook{});
-  } else if (quad_ok<DIM>(M.n[0])) {
+  } else {
     const Seg sg = make_quad_seg<DIM>(M.n[0], M.n[1], M.n[2]);
     constexpr int T = Quad<DIM>::TX * Quad<DIM>::TY;
     const LV L = lv(M);
@@ -1408,8 +1117,6 @@ void level_sm(const MgLevel& M, const LV& LC, const Kern& K, bool first, const f
     else
       launch(k_sm_q<DIM, SM_ADD, false>, quad_wave<DIM>((const void*)k_sm_q<DIM, SM_ADD, false>, sg), T,
              0, st, L, LC, sg, K, src, ec, cw, x, skip, pin, r, Hook{});
-  } else {
-    LevelOps<DIM, 1>::sm(M, LC, K, first, src, ec, cw, x, skip, pin, r, hook, st);
   }
 }
 
@@ -1580,59 +1287,6 @@ __global__ void __launch_bounds__(kT, 2) k_fcg_init(OpView<double> A, Seg sg, Fc
       S->done = 0;
       set_loop(h, 1);
     }
-  });
-}
-
-// p = z - beta p_old (p = z on the first iteration), q = A p; p.q and p.r
-// give alpha.  p alternates between two buffers by iteration parity.
-template <int DIM, int CX>
-__global__ void __launch_bounds__(kT, 2) k_fcg_dir(OpView<double> A, Seg sg, FcgState* S,
-                                                   const float* __restrict__ z, double* P0,
-                                                   double* P1, double* __restrict__ q,
-                                                   const double* __restrict__ r, double* partials,
-                                                   Loop h) {
-  pdl_enter();
-  constexpr int TX = Tile<DIM>::TX, TY = Tile<DIM>::TY;
-  __shared__ double buf[2][Rows<TY>::N][TX * CX + 2];
-  if (S->done) return;
-  const long long it = S->it;
-  const bool first = (it == 0);
-  const double beta = first ? 0.0 : S->beta;
-  double* __restrict__ pn = (it & 1) ? P1 : P0;
-  const double* __restrict__ po = (it & 1) ? P0 : P1;
-  auto val = [&](int i, int j, int k) {
-    const int64_t c = i + (int64_t)A.nx * (j + (int64_t)A.ny * k);
-    return first ? (double)z[c] : fma(-beta, po[c], (double)z[c]);
-  };
-  double acc[2] = {0.0, 0.0};
-  for_runs(sg, A.nz, [&](int tix, int tiy, int k0, int k1) {
-    march7<double, TX, TY, CX>(
-        A.nx, A.ny, A.nz, tix, tiy, k0, k1, buf, val,
-        [&](int, bool act, int i, int j, int k, double v, double w, double e, double s, double n,
-            double bo, double t) {
-          if (!act) return;
-          const int64_t c = i + (int64_t)A.nx * (j + (int64_t)A.ny * k);
-          const double aq = apply_coef(load_coef(A, i, j, k), v, w, e, s, n, bo, t);
-          pn[c] = v;
-          q[c] = aq;
-          acc[0] += v * aq;
-          acc[1] += v * r[c];
-        },
-        [](int) {});
-  });
-  reduce_last<2>(acc, partials, &S->ticket, [&](const double* tot) {
-    const double pq = tot[0], pr = tot[1];
-    const double alpha = pr / pq;
-    // A is positive definite on the space the directions live in: a
-    // non-positive p.Ap means rounding has taken over (a scale-free test; the
-    // reference's absolute 1e-30 trips on small well-converged systems)
-    if (!isfinite(pq) || !(pq > 0.0) || !isfinite(alpha)) {
-      stop_loop(S, h, kLearnedStagnated);
-      return;
-    }
-    S->pq = pq;
-    S->pr = pr;
-    S->alpha = alpha;
   });
 }
 
@@ -1857,11 +1511,11 @@ void launch_init_t(LearnedSolver* s, const FineOperator& op, Loop h, cudaStream_
          s->hist, s->hist_cap, h);
 }
 
-template <int DIM, int CX>
-void launch_dir_t(LearnedSolver* s, const FineOperator& op, Loop h, cudaStream_t st) {
-  const Seg sg = make_seg<DIM, CX>(op.A.nx, op.A.ny, op.A.nz);
-  launch(k_fcg_dir<DIM, CX>, seg_grid(sg), kT, 0, st, op.A, sg, s->S, s->z32, s->p0, s->p1, s->q,
-         s->r, s->partials, h);
+template <int DIM>
+void launch_dir_g(LearnedSolver* s, const FineOperator& op, Loop h, cudaStream_t st) {
+  const res::FaceOp<DIM> A = res::face_op<DIM>(op.A, (const double*)nullptr);
+  launch(k_fcg_dir_g<DIM>, gather_blocks(s->cells), 256, 0, st, A, (int)s->cells, s->S, s->z32, s->p0,
+         s->p1, s->q, s->r, s->partials, h);
 }
 
 void launch_init(LearnedSolver* s, const FineOperator& op, Loop h, cudaStream_t st) {
@@ -1907,12 +1561,12 @@ void launch_dir_s(LearnedSolver* s, const FineOperator& op, Loop h, cudaStream_t
 
 void launch_dir(LearnedSolver* s, const FineOperator& op, Loop h, cudaStream_t st) {
   if (op.dim == 2) {
-    if (quad_ok<2>(op.A.nx)) launch_dir_q<2>(s, op, h, st);
-    else launch_dir_t<2, 1>(s, op, h, st);
+    if (quad_ok<2>(op.A.nx) && s->cells > kGatherDirCells) launch_dir_q<2>(s, op, h, st);
+    else launch_dir_g<2>(s, op, h, st);
   } else {
     // 3D: the staged pass
     if (quad_ok<3>(op.A.nx)) launch_dir_s(s, op, h, st);
-    else launch_dir_t<3, 1>(s, op, h, st);
+    else launch_dir_g<3>(s, op, h, st);
   }
 }
 

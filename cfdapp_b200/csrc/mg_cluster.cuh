@@ -367,15 +367,7 @@ __global__ void __launch_bounds__(kClusterT, 1)
   const bool leader = T.rank_ == 0 && threadIdx.x == 0;
   const TailLevel& V = P.lv[0];
   const Share H = share_of(V.L, V.planes, T.rank_);
-  res::FaceOp<DIM> A;
-  A.A = F.A;
-  A.invd = nullptr;
-  A.nx = V.L.nx;
-  A.ny = V.L.ny;
-  A.nz = V.L.nz;
-  A.sz = (uint32_t)H.plane;
-  A.dx = V.dx;
-  A.dy = V.dy;
+  const res::FaceOp<DIM> A = res::face_op<DIM>(F.A, (const double*)nullptr);
   const double* __restrict__ b = S->b;
   double* x = S->x;
   const double abs_tol = S->abs_tol, rel_tol = S->rel_tol;

@@ -3,12 +3,12 @@
 // (one float4 / two double2 per array), so global traffic moves in 16-byte
 // vectors and the stencil reads a thread's own x-neighbours from registers
 // and its own shared-memory row.  Used where the row length is a multiple of
-// 4 and at least one tile wide; the one-cell-per-thread kernels of mg.cu
-// cover every other level.
+// 4 and at least one tile wide and the level is large; the one-cell-per-thread
+// kernels of mg_gather.cuh cover every other level.
 //
 // Tile: TX x TY threads own a (4*TX) x TY patch of an (x,y) plane and march
-// along z exactly like the generic kernels (pair-aligned plane runs).  A
-// staged plane row holds x in [x0-1, x0+4*TX] at offsets 3 .. 4*TX+4, so the
+// along z through a run of planes that starts on an even one (a coarse
+// cell's 2x2x2 children then meet inside one block).  A staged plane row holds x in [x0-1, x0+4*TX] at offsets 3 .. 4*TX+4, so the
 // thread's quad sits 16-byte aligned at 4+4*tx.
 #pragma once
 

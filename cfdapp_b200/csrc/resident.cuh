@@ -146,6 +146,20 @@ struct FaceOp {
   }
 };
 
+template <int DIM, typename V>
+__host__ __device__ inline FaceOp<DIM, V> face_op(const OpView<V>& A, const V* invd) {
+  FaceOp<DIM, V> f;
+  f.A = A;
+  f.invd = invd;
+  f.nx = A.nx;
+  f.ny = A.ny;
+  f.nz = A.nz;
+  f.sz = (uint32_t)A.nx * A.ny;
+  f.dx = fast_div(A.nx);
+  f.dy = fast_div(A.ny);
+  return f;
+}
+
 // A stored stencil matrix (stencil_solve.cuh); inv null: no preconditioner.
 // A 2D matrix's second axis is kernel space's z.
 template <int DIM>

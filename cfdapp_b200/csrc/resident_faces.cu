@@ -51,15 +51,7 @@ cfdb_status run(cfdb_context* ctx, const OpView<Value<KIND>>& V, const Value<KIN
   const int limit = cluster_limit((const void*)pcg_cluster<DIM, 8, KIND>, kClusterThreads);
   const Plan P = cg_plan(cells, (int64_t)V.nx * V.ny, ctx->num_sms, limit, sizeof(Value<KIND>));
   const uint32_t n = (uint32_t)cells;
-  FaceOp<DIM, Value<KIND>> A{};
-  A.A = V;
-  A.invd = invd;
-  A.nx = V.nx;
-  A.ny = V.ny;
-  A.nz = V.nz;
-  A.sz = (uint32_t)V.nx * V.ny;
-  A.dx = fast_div(V.nx);
-  A.dy = fast_div(V.ny);
+  const FaceOp<DIM, Value<KIND>> A = face_op<DIM>(V, invd);
   GridWords w;
   cfdb_status st = prepare_words(ctx, P, &w);
   if (st != CFDB_OK) return st;
