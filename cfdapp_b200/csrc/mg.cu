@@ -341,6 +341,7 @@ struct FcgState {
   // progress
   double b0, res, best;
   double pq, pr, alpha, beta;
+  double alpha_prev;  // of the last even iteration, whose x update waits (deferred form)
   long long it, best_it;
   int status, done;
   unsigned ticket;
@@ -1290,19 +1291,16 @@ __global__ void __launch_bounds__(kT, 2) k_fcg_init(OpView<double> A, Seg sg, Fc
   });
 }
 
-// x += alpha p; r -= alpha q; r32 = float(r); convergence, stagnation and
-// the iteration cap decide whether the loop continues.
-__global__ void k_fcg_update(int64_t n, FcgState* S, double* __restrict__ r,
-                             float* __restrict__ r32, const double* P0, const double* P1,
-                             const double* __restrict__ q, double* partials, double* hist,
-                             int64_t hcap, Loop h) {
-  pdl_enter();
-  if (S->done) return;
-  const long long it = S->it;
-  const double alpha = S->alpha;
-  const double* __restrict__ p = (it & 1) ? P1 : P0;
-  double* __restrict__ x = S->x;
-  double acc[1] = {0.0};
+// The update of this thread's cells.  XS: how many directions go into x --
+// 1 the current one, 2 the last even iteration's before it, 0 none (it waits).
+template <int XS>
+__device__ __forceinline__ double fcg_update_cells(int64_t n, double alpha, double alpha_prev,
+                                                   double* __restrict__ x, double* __restrict__ r,
+                                                   float* __restrict__ r32,
+                                                   const double* __restrict__ p,
+                                                   const double* __restrict__ pp,
+                                                   const double* __restrict__ q) {
+  double acc = 0.0;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   const int64_t tid = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   // four cells per thread in 16-byte vectors, then the remainder one by
@@ -1312,32 +1310,64 @@ __global__ void k_fcg_update(int64_t n, FcgState* S, double* __restrict__ r,
   const int64_t n4 = vec ? n / 4 : 0;
   for (int64_t g = tid; g < n4; g += stride) {
     const int64_t c = 4 * g;
-    V4<double> xv = ld4(x + c), rv = ld4(r + c);
-    const V4<double> pv = ld4(p + c), qv = ld4(q + c);
+    V4<double> xv, pv, ov, rv = ld4(r + c);
+    const V4<double> qv = ld4(q + c);
+    if (XS >= 1) xv = ld4(x + c), pv = ld4(p + c);
+    if (XS >= 2) ov = ld4(pp + c);
     V4<float> rf;
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
-      xv.v[u] = fma(alpha, pv.v[u], xv.v[u]);
+      if (XS >= 2) xv.v[u] = fma(alpha_prev, ov.v[u], xv.v[u]);
+      if (XS >= 1) xv.v[u] = fma(alpha, pv.v[u], xv.v[u]);
       const double rn = fma(-alpha, qv.v[u], rv.v[u]);
       rv.v[u] = rn;
       rf.v[u] = (float)rn;
-      acc[0] += rn * rn;
+      acc += rn * rn;
     }
-    st4(x + c, xv);
+    if (XS >= 1) st4(x + c, xv);
     st4(r + c, rv);
     st4(r32 + c, rf);
   }
   for (int64_t c = 4 * n4 + tid; c < n; c += stride) {
-    x[c] = fma(alpha, p[c], x[c]);
+    if (XS >= 2) x[c] = fma(alpha, p[c], fma(alpha_prev, pp[c], x[c]));
+    else if (XS >= 1) x[c] = fma(alpha, p[c], x[c]);
     const double rn = fma(-alpha, q[c], r[c]);
     r[c] = rn;
     r32[c] = (float)rn;
-    acc[0] += rn * rn;
+    acc += rn * rn;
   }
+  return acc;
+}
+
+// Systems from this many cells on update x every second iteration, with both
+// directions (the double buffer still holds the older one): 8 B a cell and
+// iteration less in a pass that streams at the memory's rate, and bit for
+// bit the same x.  FCG iteration (us): 256^3 756 -> 725, 160^3 323 -> 316,
+// 2048^2 241 -> 234, 1024^2 121 -> 119; below, the vectors stay in L2 and
+// the pass is as long as its latency.
+constexpr int64_t kDeferCells = 1 << 20;
+
+// x += alpha p; r -= alpha q; r32 = float(r); convergence, stagnation and
+// the iteration cap decide whether the loop continues.
+__global__ void k_fcg_update(int64_t n, FcgState* S, bool defer, double* __restrict__ r,
+                             float* __restrict__ r32, const double* P0, const double* P1,
+                             const double* __restrict__ q, double* partials, double* hist,
+                             int64_t hcap, Loop h) {
+  pdl_enter();
+  if (S->done) return;
+  const long long it = S->it;
+  const double alpha = S->alpha, prev = S->alpha_prev;
+  double* x = S->x;
+  const double* p = (it & 1) ? P1 : P0;
+  double acc[1];
+  if (!defer) acc[0] = fcg_update_cells<1>(n, alpha, 0.0, x, r, r32, p, nullptr, q);
+  else if (it & 1) acc[0] = fcg_update_cells<2>(n, alpha, prev, x, r, r32, P1, P0, q);
+  else acc[0] = fcg_update_cells<0>(n, alpha, 0.0, x, r, r32, p, nullptr, q);
   reduce_last<1>(acc, partials, &S->ticket, [&](const double* tot) {
     const double res = sqrt(tot[0]);
     const long long k = it + 1;
     S->it = k;
+    S->alpha_prev = alpha;
     S->res = res;
     if (k < hcap) hist[k] = res;
     if (!isfinite(res)) {
@@ -1357,6 +1387,17 @@ __global__ void k_fcg_update(int64_t n, FcgState* S, double* __restrict__ r,
     }
     if (k >= S->max_it) stop_loop(S, h, CFDB_SOLVER_MAX_ITERATIONS);
   });
+}
+
+// After the loop: the x update that still waits, when the last iteration
+// that updated r was an even one (its direction is P0).
+__global__ void k_fcg_last_x(int64_t n, const FcgState* S, const double* __restrict__ P0) {
+  if (!(S->it & 1)) return;
+  const double alpha = S->alpha_prev;
+  double* __restrict__ x = S->x;
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < n; c += stride)
+    x[c] = fma(alpha, P0[c], x[c]);
 }
 
 }  // namespace
@@ -1570,6 +1611,8 @@ void launch_dir(LearnedSolver* s, const FineOperator& op, Loop h, cudaStream_t s
   }
 }
 
+bool defers(const LearnedSolver* s) { return s->cells >= kDeferCells; }
+
 // One FCG iteration: V-cycle z = M r (its last kernel also forms z.q and
 // beta), direction + A p, update.  Returns the number of kernels.
 int enqueue_body(LearnedSolver* s, const FineOperator& op, Loop h, cudaStream_t st) {
@@ -1578,7 +1621,7 @@ int enqueue_body(LearnedSolver* s, const FineOperator& op, Loop h, cudaStream_t 
   const int nv = op.dim == 2 ? enqueue_cycle<2>(*s->H, s->W, s->r32, s->z32, skip, &hk, st)
                              : enqueue_cycle<3>(*s->H, s->W, s->r32, s->z32, skip, &hk, st);
   launch_dir(s, op, h, st);
-  launch(k_fcg_update, flat_grid(s->cells), 256, 0, st, s->cells, s->S, s->r, s->r32, s->p0,
+  launch(k_fcg_update, flat_grid(s->cells), 256, 0, st, s->cells, s->S, defers(s), s->r, s->r32, s->p0,
          s->p1, s->q, s->partials, s->hist, s->hist_cap, h);
   return nv + 2;
 }
@@ -1603,13 +1646,14 @@ cfdb_status run_stream_mode(cfdb_context* ctx, LearnedSolver* s, const FineOpera
 void count_bytes(LearnedSolver* s, const FineOperator& op) {
   // algorithmic bytes: the start (b, x in; r, r32 out) and per iteration the
   // V-cycle, the direction pass (z, p_old, r in; p, q out), the update (x, p,
-  // r, q in; x, r, r32 out) and the z.q read of q; face arrays when present
+  // r, q in; x, r, r32 out; a deferred x half as often, with two p) and the
+  // z.q read of q; face arrays when present
   int face_words = 0;
   for (int a = 0; a < 3; ++a) face_words += op.full[a] ? 1 : 0;
   const double n = (double)s->cells;
   s->bytes_init = n * (8.0 * (3 + face_words) + 4.0);
   s->bytes_iter = cycle_bytes(*s->H, s->W) + n * (4.0 + 8.0 * (4 + face_words)) +
-                  n * (8.0 * 6 + 4.0) + n * 8.0;
+                  n * (8.0 * (defers(s) ? 5 : 6) + 4.0) + n * 8.0;
 }
 
 // The layout of a system's FCG in one cluster (words = 0: too large, no such
@@ -1810,6 +1854,11 @@ cfdb_status learned_solve(cfdb_context* ctx, LearnedSolver* s, const FineOperato
   } else {
     CFDB_CUDA(ctx, cudaGraphLaunch(s->exec, ctx->stream));
   }
+  const bool last_x = !in_cluster && defers(s);
+  if (last_x) {
+    k_fcg_last_x<<<flat_grid(s->cells), 256, 0, ctx->stream>>>(s->cells, s->S, s->p0);
+    CFDB_CHECK_LAUNCH(ctx);
+  }
   CFDB_CUDA(ctx, cudaEventRecord(ctx->ev_k1, ctx->stream));
   CFDB_CUDA(ctx, cudaMemcpyAsync(s->S_host, s->S, sizeof(FcgState), cudaMemcpyDeviceToHost, ctx->stream));
   CFDB_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
@@ -1821,7 +1870,9 @@ cfdb_status learned_solve(cfdb_context* ctx, LearnedSolver* s, const FineOperato
   out->final_residual = hs.res;
   out->kernel_ms = ms;
   out->bytes = s->bytes_init + s->bytes_iter * (double)hs.it;
-  out->launches = in_cluster ? 1 : s->launches_init + s->launches_body * hs.it;
+  if (last_x && (hs.it & 1)) out->bytes += 8.0 * (double)s->cells;
+  out->launches =
+      in_cluster ? 1 : s->launches_init + s->launches_body * hs.it + (last_x ? 1 : 0);
   count_launch(ctx, (int)std::min<int64_t>(out->launches, 1 << 30));
   return CFDB_OK;
 }

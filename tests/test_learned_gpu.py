@@ -303,3 +303,28 @@ def test_loss_and_gradient_are_the_mean_over_samples(ctx, dim, n, samples):
                                    (2, (768, 700))])
 def test_vcycle_levels_match_oracle(ctx, dim, n):
     test_vcycle_kernels_match_oracle(ctx, dim, n)
+
+
+@pytest.mark.parametrize("n,offset", [((1024, 1024), 0), ((1025, 1025), 0), ((1024, 1024), 8),
+                                      ((105, 101, 103), 0)])
+def test_deferred_x_belongs_to_the_last_residual(ctx, n, offset):
+    """Large systems update x every second iteration: stopped after 1 to 4 iterations (odd and
+    even, aligned and unaligned x), the residual of the returned x is the recurrence's, to the
+    FP64 rounding of x seen through A (below 1e-8 of the start; bound 1e-6).  A missing or
+    doubled update changes it by the size of the residual itself."""
+    import torch
+    from cfdapp_b200.cfdb import LinearSolverSettings, POperator
+    dim, cells = len(n), int(np.prod(n))
+    b = np.random.default_rng(61).normal(size=cells)
+    b[0] = 0.0
+    op = POperator(ctx, dim, n)
+    bd = torch.tensor(b, device="cuda")
+    for its in (1, 2, 3, 4):
+        buf = torch.zeros(cells + 2, dtype=torch.float64, device="cuda")
+        torch.cuda.synchronize()
+        r = op.solve_device(bd.data_ptr(), buf.data_ptr() + offset, LinearSolverSettings(
+            preconditioner="learned_mg", absolute_tolerance=0.0, relative_tolerance=1e-30,
+            max_iterations=its))
+        assert r.iterations == its
+        assert abs(r.true_residual - r.final_residual) <= 1e-6 * r.initial_residual
+        assert float(buf[cells + 1]) == 0.0
