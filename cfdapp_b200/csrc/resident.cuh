@@ -915,7 +915,7 @@ __device__ __forceinline__ void bicgstab_run(const Op& A, uint32_t n, uint32_t l
     spmv<T, NC, PREC>(A, cells, R, team, p, P.pub, v);
     each([&](int, uint32_t lc, uint32_t) {
       const double rhv = rh[lc] * v[lc];
-      tot[0] += rhv;
+      tot[0] = fma(rh[lc], v[lc], tot[0]);  // one rounding, as in krylov_run
       tot[1] += v[lc] * v[lc];
       tot[2] += fabs(rhv);
     });
@@ -957,7 +957,7 @@ __device__ __forceinline__ void bicgstab_run(const Op& A, uint32_t n, uint32_t l
     each([&](int, uint32_t lc, uint32_t) {
       const double tsv = t[lc] * r[lc];
       tot[0] += t[lc] * t[lc];
-      tot[1] += tsv;
+      tot[1] = fma(t[lc], r[lc], tot[1]);
       tot[2] += fabs(tsv);
     });
     if (!team.reduce(tot)) return;
