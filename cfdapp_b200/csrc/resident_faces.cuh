@@ -1,0 +1,26 @@
+// Launch of the on-chip Jacobi-PCG (resident_faces.cu), instantiated for one
+// dimension and kind per translation unit: a process loads only the modules
+// it runs.  With every variant in one module the driver took 70 ms to unpack
+// it at a process's first solve; one of these takes 3-15 ms.
+#pragma once
+
+#include <cuda_runtime.h>
+
+#include <type_traits>
+
+#include "pcg_internal.cuh"
+#include "resident_launch.cuh"
+
+namespace cfdb {
+namespace res {
+
+enum { FP64 = 0, MIXED = 1, FP32 = 2 };
+template <int KIND>
+using Value = typename std::conditional<KIND == FP32, float, double>::type;
+
+template <int DIM, int KIND>
+cfdb_status pcg_on_chip(cfdb_context* ctx, const OpView<Value<KIND>>& V, const Value<KIND>* invd,
+                        const IoT<Value<KIND>>& io);
+
+}  // namespace res
+}  // namespace cfdb

@@ -62,8 +62,9 @@ inline Plan cg_plan(int64_t n, int64_t reach, int num_sms, int max_cluster, size
     const size_t words = (size_t)P.len * (team == 1 ? 3 : 2) + (halo ? 2 * (size_t)reach : 0);
     P.xs = (words + P.len) * word <= kSmemMax;
     P.smem = (words + (P.xs ? P.len : 0)) * word;
-    // a cluster's kernel has x in shared memory always
-    if (P.nc <= max_nc && P.smem <= kSmemMax && (team == 2 || P.xs)) P.team = team;
+    // a cluster's kernel and that of few cells a block have x in shared memory
+    // always (the latter fits without the neighbouring planes)
+    if (P.nc <= max_nc && P.smem <= kSmemMax && (threads == kGridThreadsLarge || P.xs)) P.team = team;
   };
   if (n <= kClusterCells && max_cluster > 0) {
     int blocks = 1;
