@@ -8,8 +8,9 @@
 //
 // Tile: TX x TY threads own a (4*TX) x TY patch of an (x,y) plane and march
 // along z through a run of planes that starts on an even one (a coarse
-// cell's 2x2x2 children then meet inside one block).  A staged plane row holds x in [x0-1, x0+4*TX] at offsets 3 .. 4*TX+4, so the
-// thread's quad sits 16-byte aligned at 4+4*tx.
+// cell's 2x2x2 children then meet inside one block).  A staged plane row
+// holds x in [x0-1, x0+4*TX] at offsets 3 .. 4*TX+4, so the thread's quad
+// sits 16-byte aligned at 4+4*tx.
 #pragma once
 
 template <int DIM>
