@@ -362,7 +362,7 @@ __global__ void __launch_bounds__(kClusterT, 1)
   const CoarsePlan& Q = to_shared(Q0, sm + plan_words<TailPlan>());
   ClusterT T = own_team(&ts);
   tail_setup<DIM>(P, Q, sm, words, T.rank_);
-  T.sync();  // every block's memory is ready for its neighbours' values
+  T.enter();  // and every block's memory is ready for its neighbours' values
   FcgState* S = F.S;
   const bool leader = T.rank_ == 0 && threadIdx.x == 0;
   const TailLevel& V = P.lv[0];

@@ -287,6 +287,9 @@ struct ClusterTeam {
                  ::: "memory");
     return true;
   }
+  // Before a block's first store into another's shared memory (a reduction
+  // makes one): every block of the cluster has started.
+  __device__ __forceinline__ void enter() { sync(); }
   // The team-wide sums of v, in every thread; a full barrier of the team.
   template <int NV>
   __device__ __forceinline__ bool reduce(double (&v)[NV]) {
@@ -365,6 +368,8 @@ struct GridTeam {
       }
     }
   }
+  // Global memory needs no block to have started.
+  __device__ __forceinline__ void enter() {}
   // published values are visible to every block afterwards
   __device__ __forceinline__ bool sync() {
     ++round;
@@ -553,6 +558,7 @@ __device__ __forceinline__ void cg_run(const Op& A, uint32_t n, uint32_t len, co
   cells.template init<T>(A, R);
   if (HALO)
     for (uint32_t q = threadIdx.x; q < len + 2 * H; q += T) sm[q] = V(0);
+  team.enter();
   V z[NC];  // z = M^-1 r between the sweeps, q = A p within an iteration
   // z of a cell for the blocks whose stencils reach it
   auto rounded = [](V v) { return MIXED ? (V)(float)v : v; };
@@ -846,6 +852,7 @@ __device__ __forceinline__ void bicgstab_run(const Op& A, uint32_t n, uint32_t l
     return team.reduce(o);
   };
   if (XS) each([&](int, uint32_t lc, uint32_t c) { xs[lc] = __ldcg(P.x + c); });
+  team.enter();
   double tot[3], one[1];
   if (!start(one)) return;
   const double b0 = sqrt(one[0]);

@@ -304,3 +304,24 @@ def test_batch_clusters_and_teams_agree(ctx, method):
         for a, c in zip(one, other):
             if a.size:
                 assert np.linalg.norm(a - c) <= 1e-8 * np.linalg.norm(c)
+
+
+@pytest.mark.parametrize("method", ["cg", "bicgstab"])
+def test_batch_clusters_with_empty_blocks(ctx, method):
+    """Cases of fewer cells than a cluster can use (9 cells: seven of the 16 blocks own none)
+    against the single-case session (linear solves to 1e-12; 1e-8 as above)."""
+    from cfdapp_b200.cfdb import Batch, LinearSolverSettings, SIMPLESettings, SimpleCase
+    ps = LinearSolverSettings(type=method, preconditioner="jacobi", absolute_tolerance=0.0,
+                              relative_tolerance=1e-12, max_iterations=200)
+    ms = LinearSolverSettings(type="bicgstab", preconditioner="none", absolute_tolerance=0.0,
+                              relative_tolerance=1e-12, max_iterations=200)
+    st = SIMPLESettings(max_iterations=3, momentum_solver=ms, pressure_solver=ps)
+    cases = [SimpleCase.cavity(2, 3), SimpleCase.channel(11, 3, 4.0, 1.0), SimpleCase.cavity(2, 40)]
+    b = Batch(ctx, cases, st)
+    for k in range(3):
+        b.set_state(k)
+    b.iterate(3)
+    res = b.results()
+    for k, case in enumerate(cases):
+        _check_against_single(ctx, case, st, b.get_state(k), res[k], bar=1e-8)
+    b.close()
