@@ -531,8 +531,9 @@ void launch_krylov(cfdb_batch* b, int mode, int comp, int record, cudaStream_t s
 
 // Whether a mode's solves run in clusters, and their kernel: FP64 ones, when
 // every case's vectors fit the shared memory of kMaxCluster blocks (65536
-// cells).  With a larger case in it the whole batch keeps to teams, which
-// share the GPU among all cases at once.
+// cells) and there are not so many cases that teams, which share the GPU
+// among all of them at once, end sooner (clusters_pay).  With a larger case in
+// it the whole batch keeps to teams.
 cfdb_status plan_clusters(cfdb_batch* b, int mode) {
   const cfdb_linear_settings& L = mode == 0 ? b->st.momentum : b->st.pressure;
   cfdb_batch::Clusters& C = b->clusters[mode];
@@ -546,6 +547,9 @@ cfdb_status plan_clusters(cfdb_batch* b, int mode) {
     C.smem = std::max(C.smem, need);
     longest = std::max(longest, (size_t)((b->cells[k] + res::kMaxCluster - 1) / res::kMaxCluster));
   }
+  std::vector<int64_t> side(b->n);
+  for (int k = 0; k < b->n; ++k) side[k] = *std::max_element(b->hc[k].G.n, b->hc[k].G.n + b->dim);
+  if (!res::clusters_pay(b->dim, b->n, side.data(), b->cells.data(), L.krylov, mode == 1)) return CFDB_OK;
   const int nc = (int)((longest + res::kClusterThreads - 1) / res::kClusterThreads);
   C.kernel = b->dim == 2 ? cluster_kernel_of<2>(L.krylov, prec, nc) : cluster_kernel_of<3>(L.krylov, prec, nc);
   if (res::cluster_limit((const void*)C.kernel, res::kClusterThreads) < res::kMaxCluster) return CFDB_OK;

@@ -7,6 +7,7 @@
 #include <map>
 #include <mutex>
 #include <utility>
+#include <vector>
 
 #include "cfdb_internal.cuh"
 #include "resident.cuh"
@@ -105,6 +106,42 @@ inline size_t cluster_smem(int64_t n, int64_t reach, int krylov, int max_nc) {
   const size_t words = krylov == 1 ? 6 * len : 4 * len + 2 * (size_t)reach;
   if (words * 8 > kSmemMax || len > (size_t)max_nc * kClusterThreads) return 0;
   return words * 8;
+}
+
+// Whether clusters of kMaxCluster blocks, one per case and kClustersAtOnce at
+// a time, end the solves of a batch sooner than block teams, which advance
+// all cases together.  side, cells: each case's longest side and cells.
+//
+// A solve's iterations: in proportion to its side for the p' systems
+// (poisson), alike for the diagonally dominant momentum systems.  The time of
+// an iteration, as a share of a team's in a small batch (about 25 us), from
+// solves of 4 to 64 equal cases:
+//   cluster  CG 0.2 up to 2 cells a thread (48^2 0.20, 128^2 0.18), then 0.33
+//            (192^2; 33^3 0.28) to 0.41 (256^2); BiCGSTAB 0.31 (128^2 0.30), 0.39, 0.46
+//   teams    1 until the batch's vectors fill L2, then in proportion to its
+//            cells: 1.2 at 0.85 M, 1.4 at 1.05 M, 2.4 at 1.8 M, 3.2 at 2.4 M
+// p' solves of an outer iteration (ms, clusters / teams): 128^2 x 16 9.4 /
+// 17.7, x 32 15.6 / 18.6, x 48 21.9 / 20.0, x 64 31.1 / 22.9; 48^2 x 64 9.7 /
+// 4.9; 256^2 x 32 67.5 / 99.4.  Momentum: 48^2 x 16 1.19 / 1.18, x 64 4.0 /
+// 1.2; 256^2 x 16 1.9 / 2.2.
+constexpr int kClustersAtOnce = 7;
+inline bool clusters_pay(int dim, int ncases, const int64_t* side, const int64_t* cells, int krylov,
+                         bool poisson) {
+  double all = 0.0, longest = 0.0;
+  double busy[kClustersAtOnce] = {};
+  std::vector<double> cost(ncases);
+  for (int k = 0; k < ncases; ++k) {
+    const double its = poisson ? (double)side[k] : 1.0, n = (double)cells[k];
+    const bool few = cells[k] <= 2 * kMaxCluster * kClusterThreads;
+    const double cg = few ? 0.2 : (0.23 + 2.8e-6 * n) * (dim == 3 ? 0.85 : 1.0);
+    cost[k] = its * (krylov == 1 ? (few ? 0.31 : 0.30 + 2.5e-6 * n) : cg);
+    all += n;
+    longest = std::max(longest, its);
+  }
+  const double teams = longest * std::max(1.0 + 0.24e-6 * all, 1.35e-6 * all);
+  std::sort(cost.begin(), cost.end(), [](double a, double b) { return a > b; });
+  for (double c : cost) *std::min_element(busy, busy + kClustersAtOnce) += c;
+  return *std::max_element(busy, busy + kClustersAtOnce) < teams;
 }
 
 // Largest cluster size (16, 8, ... 1; 0 on failure) `fn` can run at with the

@@ -71,3 +71,37 @@ def test_cluster_solves_enter_the_team_first(tmp_path, sym, run):
     ops, status = _run(tmp_path, KRYLOV.replace("RUN", run).replace("SYM", str(sym)))
     assert status == "0"  # converged
     assert ops[0] == "e", ops
+
+
+# measured solve stages of one outer iteration on the GPU (ms, clusters and teams): dimension,
+# side, cases, method, p' system or momentum
+STAGES = [(2, 48, 7, 0, 1, 0.98, 4.7), (2, 48, 64, 0, 1, 9.7, 4.9), (2, 96, 24, 0, 1, 8.9, 13.8),
+          (2, 96, 64, 0, 1, 22.2, 14.5), (2, 128, 16, 0, 1, 9.4, 17.7), (2, 128, 32, 0, 1, 15.6, 18.6),
+          (2, 128, 64, 0, 1, 31.1, 22.9), (2, 192, 16, 0, 1, 23.9, 27.0),
+          (2, 256, 16, 0, 1, 40.4, 46.7), (2, 256, 32, 0, 1, 67.5, 99.4),
+          (3, 16, 64, 0, 1, 5.8, 3.9), (3, 33, 16, 0, 1, 8.8, 10.9), (3, 33, 32, 0, 1, 14.6, 17.3),
+          (3, 33, 48, 0, 1, 20.5, 21.9),
+          (2, 128, 32, 1, 1, 39.4, 29.1), (2, 128, 16, 1, 1, 23.6, 27.7),
+          (2, 48, 7, 1, 0, 0.41, 1.15), (2, 48, 32, 1, 0, 1.98, 1.18), (2, 128, 64, 1, 0, 4.09, 2.17),
+          (2, 256, 16, 1, 0, 1.90, 2.21), (2, 256, 32, 1, 0, 3.18, 3.98),
+          (3, 24, 32, 1, 0, 3.49, 2.24), (3, 24, 8, 1, 0, 1.40, 2.16)]
+
+
+def test_batches_take_clusters_where_they_were_faster(tmp_path):
+    """The choice between one cluster per case and block teams, against both sides measured."""
+    rows = "".join(f"{{{d},{s},{c},{k},{p}}}," for d, s, c, k, p, _, _ in STAGES)
+    got = _run(tmp_path, r"""
+#include "device_on_host.h"
+#include "resident_launch.cuh"
+#include <cstdio>
+int main() {
+  const int rows[][5] = {""" + rows + r"""};
+  for (auto& r : rows) {
+    const int64_t n = r[0] == 2 ? (int64_t)r[1] * r[1] : (int64_t)r[1] * r[1] * r[1];
+    std::vector<int64_t> side(r[2], r[1]), cells(r[2], n);
+    printf("%d ", (int)cfdb::res::clusters_pay(r[0], r[2], side.data(), cells.data(), r[3], r[4]));
+  }
+}
+""")
+    for row, pay in zip(STAGES, got):
+        assert (pay == "1") == (row[5] < row[6]), row
