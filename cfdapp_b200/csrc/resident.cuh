@@ -995,7 +995,7 @@ __device__ __forceinline__ void bicgstab_run(const Op& A, uint32_t n, uint32_t l
       r[lc] = rn;
       const double rhr = rh[lc] * rn;
       tot[0] += rn * rn;
-      tot[1] += rhr;
+      tot[1] = fma(rh[lc], rn, tot[1]);
       tot[2] += fabs(rhr);
     });
     if (!team.reduce(tot)) return;

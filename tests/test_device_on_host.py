@@ -105,3 +105,39 @@ int main() {
 """)
     for row, pay in zip(STAGES, got):
         assert (pay == "1") == (row[5] < row[6]), row
+
+
+def test_bicgstab_dot_products_round_once(tmp_path):
+    """The three dot products of an iteration -- (rHat, v), (t, s) and (rHat, r) -- as sums of
+    fused multiply-adds: a single-thread team sees the sums and the vectors they are of."""
+    team = r"""
+struct Team {
+  static constexpr bool kGlobal = false;
+  const double *rh, *v, *r, *t;
+  int n, triple = 0, bad = 0, seen = 0;
+  int rank() const { return 0; }
+  void enter() {}
+  bool sync() { return true; }
+  double dot(const double* a, const double* b) const {
+    double s = 0.0;
+    for (int c = 0; c < n; ++c) s = fma(a[c], b[c], s);
+    return s;
+  }
+  template <int NV> bool reduce(double (&o)[NV]) {
+    if (NV != 3) return true;
+    const double want[3] = {dot(rh, v), dot(t, r), dot(rh, r)};
+    ++seen;
+    bad += o[triple == 0 ? 0 : 1] != want[triple];
+    triple = (triple + 1) % 3;
+    return true;
+  }
+  double remote(const double* q, const double*, uint32_t c) const { return q[c]; }
+};
+int main() {"""
+    src = KRYLOV.replace(KRYLOV[KRYLOV.index("struct Team"):KRYLOV.index("int main() {") + 12], team)
+    src = src.replace("SYM", "0").replace("RUN", r"""
+  T.n = n; T.r = sm + n; T.rh = sm + 2 * n; T.v = sm + 3 * n; T.t = sm + 4 * n;
+  res::bicgstab_run<1, 0, true, false>(res::band_op<2>(M), (uint32_t)n, (uint32_t)n, P, T, sm);
+""").replace(r'printf("%s %d\n", T.ops.c_str(), (int)out[0]);', r'printf("%d %d\n", T.seen, T.bad);')
+    seen, bad = _run(tmp_path, src)
+    assert int(seen) >= 9 and bad == "0", (seen, bad)
