@@ -12,7 +12,7 @@ cfdb_status run(cfdb_context* ctx, const StencilMatrix& M, int krylov, const Io&
   *taken = false;
   int limit = 0;  // asked for where a cluster may take the system
   if (krylov == 1 && M.n <= kBicgClusterCells) limit = bicgstab_cluster_limit<DIM>();
-  if (krylov != 1 && M.n <= kClusterCells) limit = cg_cluster_limit<DIM>();
+  if (krylov != 1 && M.n <= cluster_cells(DIM)) limit = cg_cluster_limit<DIM>();
   const BandOp<DIM> A = band_op<DIM>(M);
   const Plan P = krylov == 1 ? bicgstab_plan(M.n, ctx->num_sms, limit)
                              : cg_plan(M.n, A.sz, ctx->num_sms, limit);

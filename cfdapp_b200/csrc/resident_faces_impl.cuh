@@ -36,7 +36,7 @@ template <int DIM, int KIND>
 cfdb_status pcg_on_chip(cfdb_context* ctx, const OpView<Value<KIND>>& V, const Value<KIND>* invd,
                         const IoT<Value<KIND>>& io) {
   const int64_t cells = (int64_t)V.nx * V.ny * V.nz;
-  const int limit = cells <= kClusterCells
+  const int limit = cells <= cluster_cells(DIM)
                         ? cluster_limit((const void*)pcg_cluster<DIM, 8, KIND>, kClusterThreads)
                         : 0;
   const Plan P = cg_plan(cells, (int64_t)V.nx * V.ny, ctx->num_sms, limit, sizeof(Value<KIND>));

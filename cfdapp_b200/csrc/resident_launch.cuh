@@ -24,7 +24,7 @@ constexpr int kClusterNC = 8, kGridNC = 14;  // most cells per thread
 constexpr int kGridThreadsSmall = 512, kGridThreadsLarge = 1024;
 constexpr uint32_t kGridSmallCells = 2048;  // cells per block
 
-// As kClusterCells; a BiCGSTAB iteration (us, cluster / grid): 129^2 12.2 / 13,
+// As cluster_cells; a BiCGSTAB iteration (us, cluster / grid): 129^2 12.2 / 13,
 // 181^2 13.4 / 13.5, 33^3 16.7 / 17.
 constexpr int64_t kBicgClusterCells = 32768;
 
@@ -40,15 +40,19 @@ struct Plan {
 };
 
 // Cells a cluster takes before the whole GPU is the faster team, by the time
-// of a CG iteration (us, cluster / grid): 129^2 4.7 / 6.6, 181^2 (32 761 cells)
-// 5.6 / 6.6, 33^3 7.5 / 7.2, 250^2 8.0 / 6.7, 40^3 10.2 / 6.7.
-constexpr int64_t kClusterCells = 36864;
+// of an FP64 CG iteration (us, cluster / grid).  2D: 150^2 4.9 / 5.9, 181^2
+// (32 761 cells: the last with four a thread) 5.65 / 5.92, 182^2 6.05 / 5.74,
+// 190^2 6.11 / 5.76.  3D, whose ranges read larger planes: 26^3 5.4 / 6.2,
+// 29^3 6.1 / 6.4, 30^3 6.7 / 6.4, 33^3 7.3 / 6.3.  (Mixed precision meets at
+// the same places within 5 %.)
+constexpr int64_t cluster_cells(int dim) { return dim == 2 ? 32768 : 25600; }
 
 // Layout of the CG of n cells.  A cluster's size grows with the system until every
 // block has one cell per thread; per iteration (us, streaming kernel before):
 // 40x33 2.7 (18.6), 129^2 4.7 (13.0), 512^2 8.0 (20.9), 64^3 9.6 (19.5),
 // 96^3 16.7 (29.3), 128^3 31.8 (44.7); the last two keep no neighbouring
-// planes.  `reach`: cells the stencil reaches (a plane).
+// planes.  `reach`: cells the stencil reaches (a plane); max_cluster: 0 past
+// cluster_cells.
 inline Plan cg_plan(int64_t n, int64_t reach, int num_sms, int max_cluster, size_t word = 8) {
   Plan P;
   auto fill = [&](int team, int blocks, int max_nc, bool halo) {
@@ -67,7 +71,7 @@ inline Plan cg_plan(int64_t n, int64_t reach, int num_sms, int max_cluster, size
     // always (the latter fits without the neighbouring planes)
     if (P.nc <= max_nc && P.smem <= kSmemMax && (threads == kGridThreadsLarge || P.xs)) P.team = team;
   };
-  if (n <= kClusterCells && max_cluster > 0) {
+  if (max_cluster > 0) {
     int blocks = 1;
     while (blocks < max_cluster && (int64_t)blocks * kClusterThreads < n) blocks *= 2;
     fill(1, blocks, kClusterNC, true);

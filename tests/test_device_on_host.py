@@ -141,3 +141,25 @@ int main() {"""
 """).replace(r'printf("%s %d\n", T.ops.c_str(), (int)out[0]);', r'printf("%d %d\n", T.seen, T.bad);')
     seen, bad = _run(tmp_path, src)
     assert int(seen) >= 9 and bad == "0", (seen, bad)
+
+
+# measured CG iterations on the GPU (us, cluster and grid): dimension, cells, plane
+LINE = [(2, 22500, 150, 4.9, 5.9), (2, 32761, 181, 5.65, 5.92), (2, 33124, 182, 6.05, 5.74),
+        (2, 36100, 190, 6.11, 5.76), (3, 24389, 841, 6.1, 6.4), (3, 27000, 900, 6.7, 6.4),
+        (3, 35937, 1089, 7.3, 6.3)]
+
+
+def test_cg_takes_the_team_that_was_faster(tmp_path):
+    got = _run(tmp_path, r"""
+#include "device_on_host.h"
+#include "resident_launch.cuh"
+#include <cstdio>
+using namespace cfdb::res;
+int main() {
+  const int rows[][3] = {""" + "".join(f"{{{d},{n},{h}}}," for d, n, h, _, _ in LINE) + r"""};
+  for (auto& r : rows)
+    printf("%d ", cg_plan(r[1], r[2], 148, r[1] <= cluster_cells(r[0]) ? 16 : 0).team);
+}
+""")
+    for row, team in zip(LINE, got):
+        assert team == ("1" if row[3] < row[4] else "2"), row
