@@ -38,6 +38,25 @@ cfdb_status ensure_partials(cfdb_context* ctx, size_t doubles) {
   return CFDB_OK;
 }
 
+cudaError_t CallScratch::get(size_t bytes, void** out) {
+  cudaError_t e = cudaSuccess;
+  if (bytes > kScratchKept) {
+    e = cudaMalloc(&own_, bytes);
+    *out = own_;
+  } else {
+    if (ctx_->scratch_cap < bytes) {
+      cudaFree(ctx_->scratch);
+      ctx_->scratch = nullptr;
+      ctx_->scratch_cap = 0;
+      e = cudaMalloc(&ctx_->scratch, bytes);
+      if (e == cudaSuccess) ctx_->scratch_cap = bytes;
+    }
+    *out = ctx_->scratch;
+  }
+  if (e != cudaSuccess) cudaGetLastError();  // the caller may ask for less
+  return e;
+}
+
 }  // namespace cfdb
 
 using namespace cfdb;
@@ -118,6 +137,7 @@ void cfdb_destroy(cfdb_context* ctx) {
   cudaSetDevice(ctx->device);
   if (ctx->stream) cudaStreamSynchronize(ctx->stream);
   cudaFree(ctx->partials);
+  cudaFree(ctx->scratch);
   cudaFree(ctx->sync_words);
   cudaFree(ctx->scalars);
   if (ctx->scalars_host) cudaFreeHost(ctx->scalars_host);

@@ -22,6 +22,8 @@ struct cfdb_context {
   unsigned* sync_words = nullptr;  // [0] arrival count [1] generation [2] error flag
   double* scalars = nullptr;       // device scalars written by kernels (64 doubles)
   double* scalars_host = nullptr;  // pinned mirror
+  void* scratch = nullptr;         // vectors of a training step (kept up to kScratchKept)
+  size_t scratch_cap = 0;          // bytes
   cudaEvent_t ev_start = nullptr, ev_stop = nullptr;
   cudaEvent_t ev_k0 = nullptr, ev_k1 = nullptr;  // around persistent kernel launches
   // Learned-preconditioner weights of this context (owned; see mg.cu).
@@ -36,6 +38,23 @@ cfdb_status cuda_error(cfdb_context* ctx, cudaError_t err, const char* what, con
                        int line);
 // Grows the per-block partials scratch to at least `doubles` entries.
 cfdb_status ensure_partials(cfdb_context* ctx, size_t doubles);
+
+// Device memory for the duration of one call on the context's stream, which
+// has ended when this goes.  What the context holds between calls is at most
+// kScratchKept, one for all its operators; a larger piece is freed again.
+constexpr size_t kScratchKept = (size_t)256 << 20;
+class CallScratch {
+ public:
+  explicit CallScratch(cfdb_context* ctx) : ctx_(ctx) {}
+  ~CallScratch() { cudaFree(own_); }
+  CallScratch(const CallScratch&) = delete;
+  CallScratch& operator=(const CallScratch&) = delete;
+  cudaError_t get(size_t bytes, void** out);
+
+ private:
+  cfdb_context* ctx_;
+  void* own_ = nullptr;
+};
 
 inline void count_launch(cfdb_context* ctx, int n = 1) { ctx->launches += n; }
 

@@ -1495,8 +1495,6 @@ struct LearnedSolver {
   cudaGraphExec_t exec = nullptr;
   int64_t launches_init = 0, launches_body = 0;
   double bytes_init = 0, bytes_iter = 0;
-  void* scratch = nullptr;
-  size_t scratch_bytes = 0;
 
   void free_graph() {
     if (exec) cudaGraphExecDestroy(exec);
@@ -1516,9 +1514,6 @@ struct LearnedSolver {
     S = nullptr;
     hist = nullptr;
     hist_cap = 0;
-    cudaFree(scratch);
-    scratch = nullptr;
-    scratch_bytes = 0;
     if (S_host) cudaFreeHost(S_host);
     S_host = nullptr;
     if (cap) cudaStreamDestroy(cap);
@@ -1874,18 +1869,6 @@ cfdb_status learned_solve(cfdb_context* ctx, LearnedSolver* s, const FineOperato
   out->launches =
       in_cluster ? 1 : s->launches_init + s->launches_body * hs.it + (last_x ? 1 : 0);
   count_launch(ctx, (int)std::min<int64_t>(out->launches, 1 << 30));
-  return CFDB_OK;
-}
-
-cfdb_status learned_scratch(cfdb_context* ctx, LearnedSolver* s, size_t bytes, void** out) {
-  if (s->scratch_bytes < bytes) {
-    cudaFree(s->scratch);
-    s->scratch = nullptr;
-    s->scratch_bytes = 0;
-    CFDB_CUDA(ctx, cudaMalloc(&s->scratch, bytes));
-    s->scratch_bytes = bytes;
-  }
-  *out = s->scratch;
   return CFDB_OK;
 }
 

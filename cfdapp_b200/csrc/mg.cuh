@@ -120,9 +120,6 @@ cfdb_status learned_solve(cfdb_context* ctx, LearnedSolver* s, const FineOperato
 // The solver's hierarchy for `op`, built or refreshed as a solve would.
 cfdb_status learned_hierarchy(cfdb_context* ctx, LearnedSolver* s, const FineOperator& op,
                               uint64_t version, const MgHierarchy** out);
-// At least `bytes` of device memory that the solver keeps (grown as needed)
-// for passes of its own operator, one at a time.
-cfdb_status learned_scratch(cfdb_context* ctx, LearnedSolver* s, size_t bytes, void** out);
 // Copies the first m residual-history entries of the last solve to the host.
 cfdb_status learned_history(cfdb_context* ctx, LearnedSolver* s, double* host, int64_t m);
 

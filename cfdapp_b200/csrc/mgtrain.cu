@@ -18,7 +18,7 @@
 // grids, where a pass over one sample is all launch latency, so every pass
 // covers all samples of the step at once (grid.y = sample, each sample's
 // vectors back to back; the samples go in chunks where they would need more
-// than kScratchBytes): at 128^2 and 8 samples a step takes
+// than the context keeps for a step): at 128^2 and 8 samples a step takes
 // 0.51 ms, sample by sample it took 4.67.
 #include <cuda_runtime.h>
 
@@ -353,9 +353,6 @@ __global__ void t_clear_pin(int64_t n, int64_t pin, int samples, float* v) {
 
 // ------------------------------------------------------------------ driver
 
-// Scratch of a step; more samples than fit it go in chunks.
-constexpr size_t kScratchBytes = (size_t)256 << 20;
-
 struct Trainer {
   cfdb_context* ctx;
   const MgHierarchy& H;
@@ -524,10 +521,13 @@ cfdb_status cfdb_mg_loss_grad(cfdb_context* ctx, cfdb_poperator* op, int nsample
   // as many samples at once as fit the scratch
   Trainer T(ctx, *H, W, pin, 1);
   const size_t each = T.layout(nullptr, nsamples);
-  T.samples = (int)std::min<size_t>({(size_t)nsamples, std::max<size_t>(1, kScratchBytes / each), 65535});
+  T.samples = (int)std::min<size_t>({(size_t)nsamples, std::max<size_t>(1, kScratchKept / each), 65535});
+  CallScratch memory(ctx);
   void* scratch = nullptr;
-  st = learned_scratch(ctx, solver, T.layout(nullptr, nsamples), &scratch);
-  if (st != CFDB_OK) return set_error(ctx, CFDB_ERR_OUT_OF_MEMORY, "training buffers");
+  while (memory.get(T.layout(nullptr, nsamples), &scratch) != cudaSuccess) {
+    if (T.samples == 1) return set_error(ctx, CFDB_ERR_OUT_OF_MEMORY, "training buffers");
+    T.samples = (T.samples + 1) / 2;
+  }
   T.layout((char*)scratch, nsamples);
   st = T.upload_levels();
   if (st != CFDB_OK) return st;

@@ -535,7 +535,9 @@ CFDB_API cfdb_status cfdb_mg_apply(cfdb_context* ctx, cfdb_poperator* op, const 
  * differentiation: grad_kernels[16*27] (tied taps t and 26-t receive the same
  * summed value; 2D sets use taps 9..17) and grad_coarse[16], per level that
  * owns weights (levels deeper than the weight set's count add into the last).
- * Either gradient pointer may be NULL. */
+ * Either gradient pointer may be NULL.  The step's vectors take up to 256 MB
+ * of device memory that the context keeps until it is destroyed (one piece
+ * for all its operators); a sample that needs more has it for the call. */
 CFDB_API cfdb_status cfdb_mg_loss_grad(cfdb_context* ctx, cfdb_poperator* op, int nsamples,
                                        const float* e_host, double* loss, double* grad_kernels,
                                        double* grad_coarse);

@@ -328,3 +328,27 @@ def test_deferred_x_belongs_to_the_last_residual(ctx, n, offset):
         assert r.iterations == its
         assert abs(r.true_residual - r.final_residual) <= 1e-6 * r.initial_residual
         assert float(buf[cells + 1]) == 0.0
+
+
+@pytest.mark.parametrize("n,samples", [((64, 64, 64), 15), ((2304, 2300), 1)])
+def test_training_steps_leave_bounded_memory(n, samples):
+    """A step's vectors (250 MB for 15 samples of 64^3, 480 MB for one of 2304x2300) stay with
+    the context up to 256 MB, not with each operator: once one operator has made a step, another
+    that is ready to solve takes no more than 32 MB for its own."""
+    import torch
+    from cfdapp_b200.cfdb import Context, POperator
+    ctx = Context(0)
+    dim, cells = len(n), int(np.prod(n))
+    e = np.random.default_rng(71).normal(size=(samples, cells)).astype(np.float32)
+    b = np.random.default_rng(72).normal(size=cells)
+    b[0] = 0.0
+    ops = [POperator(ctx, dim, n) for _ in range(2)]
+    for op in ops:
+        op.solve(b, _settings(max_iterations=1))
+    ops[0].mg_loss_grad(e)
+    before = torch.cuda.mem_get_info()[0]
+    ops[1].mg_loss_grad(e)
+    assert before - torch.cuda.mem_get_info()[0] <= 32 << 20
+    for op in ops:
+        op.close()
+    ctx.close()
