@@ -383,6 +383,7 @@ __global__ void __launch_bounds__(kClusterT, 1)
     put(sm + V.ou, H, V.planes, T.rank_, t, kl, t == pin ? 0.f : __ldg(V.L.isq + c) * (float)rn);
   };
   auto stop = [&](int status, long long it, double res) {
+    cp_wait<0>();  // no copy of the coarse levels is in flight when the block leaves
     if (leader) {
       S->it = it;
       S->res = res;

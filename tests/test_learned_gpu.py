@@ -352,3 +352,22 @@ def test_training_steps_leave_bounded_memory(n, samples):
     for op in ops:
         op.close()
     ctx.close()
+
+
+@pytest.mark.parametrize("n", [(40, 33), (21, 20, 19)])
+def test_small_learned_solves_that_end_at_once(ctx, n):
+    """A small system's solve that stops before its first V-cycle (zero right-hand side; a start
+    that meets the tolerance) while its coarse levels are still being fetched, each followed by a
+    whole solve: that one's solution is the one found before them, bit for bit."""
+    from cfdapp_b200.cfdb import POperator
+    dim, cells = len(n), int(np.prod(n))
+    b = np.random.default_rng(81).normal(size=cells)
+    b[0] = 0.0
+    op = POperator(ctx, dim, n)
+    ref = op.solve(b, _settings())
+    for _ in range(20):
+        zero = op.solve(np.zeros(cells), _settings())
+        assert zero.status == "Converged" and zero.iterations == 0
+        loose = op.solve(b, _settings(absolute_tolerance=1e6))
+        assert loose.status == "Converged" and loose.iterations == 0
+        assert np.array_equal(op.solve(b, _settings()).solution, ref.solution)
