@@ -1030,7 +1030,7 @@ GLevel gcoarse(const LV& C) {
   G.L = C;
   G.dx = res::fast_div(C.nx);
   G.dy = res::fast_div(C.ny);
-  G.n = C.nx * C.ny * C.nz;
+  G.n = (uint32_t)C.nx * C.ny * C.nz;
   return G;
 }
 
@@ -1042,11 +1042,11 @@ void level_res(const MgLevel& M, const LV& LC, const float* x, const float* ec, 
     const int g = gather_blocks(M.cells);
     if (rc) {
       const GLevel C = gcoarse(LC);
-      launch(k_restrict_g<DIM>, gather_blocks(C.n), 256, 0, st, G, C, x, r, rc, (int)skip);
+      launch(k_restrict_g<DIM>, gather_blocks(C.n), 256, 0, st, G, C, x, r, rc, (uint32_t)skip);
     } else if (ec) {
-      launch(k_resid_g<DIM, true>, g, 256, 0, st, G, LC, x, ec, cw, r, res, (int)skip);
+      launch(k_resid_g<DIM, true>, g, 256, 0, st, G, LC, x, ec, cw, r, res, (uint32_t)skip);
     } else {
-      launch(k_resid_g<DIM, false>, g, 256, 0, st, G, LC, x, ec, cw, r, res, (int)skip);
+      launch(k_resid_g<DIM, false>, g, 256, 0, st, G, LC, x, ec, cw, r, res, (uint32_t)skip);
     }
   } else if (DIM == 3 && quad_ok<DIM>(M.n[0])) {
     const Seg sg = make_quad_seg<3>(M.n[0], M.n[1], M.n[2]);
@@ -1086,11 +1086,11 @@ void level_sm(const MgLevel& M, const LV& LC, const Kern& K, bool first, const f
     const GLevel G = glevel(M);
     const int g = gather_blocks(M.cells);
     if (first)
-      launch(k_first_g<DIM>, g, 256, 0, st, G, K, src, x, (int)skip);
+      launch(k_first_g<DIM>, g, 256, 0, st, G, K, src, x, (uint32_t)skip);
     else if (hook)
-      launch(k_smooth_g<DIM, true>, g, 256, 0, st, G, LC, K, src, ec, cw, x, (int)pin, r, *hook);
+      launch(k_smooth_g<DIM, true>, g, 256, 0, st, G, LC, K, src, ec, cw, x, (uint32_t)pin, r, *hook);
     else
-      launch(k_smooth_g<DIM, false>, g, 256, 0, st, G, LC, K, src, ec, cw, x, (int)pin, r, Hook{});
+      launch(k_smooth_g<DIM, false>, g, 256, 0, st, G, LC, K, src, ec, cw, x, (uint32_t)pin, r, Hook{});
   } else if (DIM == 3 && quad_ok<DIM>(M.n[0])) {
     const Seg sg = make_quad_seg<3>(M.n[0], M.n[1], M.n[2]);
     constexpr int T = PlaneTile::T;
@@ -1550,7 +1550,7 @@ void launch_init_t(LearnedSolver* s, const FineOperator& op, Loop h, cudaStream_
 template <int DIM>
 void launch_dir_g(LearnedSolver* s, const FineOperator& op, Loop h, cudaStream_t st) {
   const res::FaceOp<DIM> A = res::face_op<DIM>(op.A, (const double*)nullptr);
-  launch(k_fcg_dir_g<DIM>, gather_blocks(s->cells), 256, 0, st, A, (int)s->cells, s->S, s->z32, s->p0,
+  launch(k_fcg_dir_g<DIM>, gather_blocks(s->cells), 256, 0, st, A, (uint32_t)s->cells, s->S, s->z32, s->p0,
          s->p1, s->q, s->r, s->partials, h);
 }
 

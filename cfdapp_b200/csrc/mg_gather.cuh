@@ -16,7 +16,7 @@
 struct GLevel {
   LV L;
   res::FastDiv dx, dy;
-  int n;
+  uint32_t n;
 };
 
 GLevel glevel(const MgLevel& M) {
@@ -24,7 +24,7 @@ GLevel glevel(const MgLevel& M) {
   G.L = lv(M);
   G.dx = res::fast_div(M.n[0]);
   G.dy = res::fast_div(M.n[1]);
-  G.n = (int)M.cells;
+  G.n = (uint32_t)M.cells;
   return G;
 }
 
@@ -33,19 +33,13 @@ int gather_blocks(int64_t n) {
   return (int)std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, kMaxBlocks));
 }
 
-template <class F>
-__device__ __forceinline__ void gather_cells(int n, int nx, int ny, res::FastDiv dx, res::FastDiv dy, F f) {
-  for (int c = blockIdx.x * 256 + threadIdx.x; c < n; c += gridDim.x * 256) {
-    const uint32_t row = dx.div((uint32_t)c), k = dy.div(row);
-    f(c, (int)(c - row * (uint32_t)nx), (int)(row - k * (uint32_t)ny), (int)k);
-  }
-}
+using res::gather_cells;
 
 // Couplings of a cell (coef() with 32-bit indices).
 template <int DIM>
-__device__ __forceinline__ C7 gather_coef(const LV& L, int c, int j, int k) {
+__device__ __forceinline__ C7 gather_coef(const LV& L, uint32_t c, int j, int k) {
   C7 o;
-  const int row = j + L.ny * k;
+  const uint32_t row = j + L.ny * k;
   o.xl = L.fx[c + row];
   o.xh = L.fx[c + row + 1];
   o.yl = DIM == 3 ? L.fy[c + L.nx * k] : 0.f;
@@ -58,7 +52,7 @@ __device__ __forceinline__ C7 gather_coef(const LV& L, int c, int j, int k) {
 
 // (A v)(c); val(q, di, dj, dk) is v at cell q = c + offset.
 template <int DIM, class Val>
-__device__ __forceinline__ float gather_lap(const LV& L, int c, int i, int j, int k, Val val) {
+__device__ __forceinline__ float gather_lap(const LV& L, uint32_t c, int i, int j, int k, Val val) {
   const int plane = L.nx * L.ny;
   auto at = [&](bool in, int off, int di, int dj, int dk) {
     const float v = val(in ? c + off : c, in ? di : 0, in ? dj : 0, in ? dk : 0);
@@ -74,7 +68,7 @@ __device__ __forceinline__ float gather_lap(const LV& L, int c, int i, int j, in
 
 // sum_o K[o] u(c + o), taps in (dz, dy, dx) order.
 template <int DIM, class U>
-__device__ __forceinline__ float gather_conv(const LV& L, const Kern& K, int c, int i, int j, int k, U u) {
+__device__ __forceinline__ float gather_conv(const LV& L, const Kern& K, uint32_t c, int i, int j, int k, U u) {
   float sum = 0.f;
 #pragma unroll
   for (int dk = -1; dk <= 1; ++dk) {
@@ -82,7 +76,7 @@ __device__ __forceinline__ float gather_conv(const LV& L, const Kern& K, int c, 
 #pragma unroll
     for (int dj = (DIM == 2 ? 0 : -1); dj <= (DIM == 2 ? 0 : 1); ++dj) {
       const bool yin = zin && (DIM == 2 || (j + dj >= 0 && j + dj < L.ny));
-      const int q = c + dk * L.nx * L.ny + dj * L.nx;
+      const uint32_t q = c + dk * L.nx * L.ny + dj * L.nx;
 #pragma unroll
       for (int di = -1; di <= 1; ++di) {
         const bool in = yin && i + di >= 0 && i + di < L.nx;
@@ -101,11 +95,11 @@ __device__ __forceinline__ int gather_parent(const LV& C, int i, int j, int k) {
 // x = D^-1/2 (W * (D^-1/2 r)), r[skip] read as 0
 template <int DIM>
 __global__ void __launch_bounds__(256) k_first_g(GLevel G, Kern K, const float* __restrict__ r,
-                                                 float* __restrict__ x, int skip) {
+                                                 float* __restrict__ x, uint32_t skip) {
   pdl_enter();
   const LV& L = G.L;
-  gather_cells(G.n, L.nx, L.ny, G.dx, G.dy, [&](int c, int i, int j, int k) {
-    const float s = gather_conv<DIM>(L, K, c, i, j, k, [&](int q) {
+  gather_cells(G.n, L.nx, L.ny, G.dx, G.dy, [&](uint32_t c, int i, int j, int k) {
+    const float s = gather_conv<DIM>(L, K, c, i, j, k, [&](uint32_t q) {
       const float v = r[q] * L.isq[q];
       return q == skip ? 0.f : v;
     });
@@ -117,10 +111,10 @@ __global__ void __launch_bounds__(256) k_first_g(GLevel G, Kern K, const float* 
 template <int DIM>
 __global__ void __launch_bounds__(256) k_restrict_g(GLevel G, GLevel C, const float* __restrict__ x,
                                                     const float* __restrict__ r,
-                                                    float* __restrict__ rc, int skip) {
+                                                    float* __restrict__ rc, uint32_t skip) {
   pdl_enter();
   const LV& L = G.L;
-  gather_cells(C.n, C.L.nx, C.L.ny, C.dx, C.dy, [&](int qc, int ci, int cj, int ck) {
+  gather_cells(C.n, C.L.nx, C.L.ny, C.dx, C.dy, [&](uint32_t qc, int ci, int cj, int ck) {
     float sum = 0.f;
 #pragma unroll
     for (int u = 0; u < 2; ++u)
@@ -130,8 +124,8 @@ __global__ void __launch_bounds__(256) k_restrict_g(GLevel G, GLevel C, const fl
         for (int t = 0; t < 2; ++t) {
           const int i = 2 * ci + t, j = DIM == 3 ? 2 * cj + v : 0, k = 2 * ck + u;
           if (i < L.nx && j < L.ny && k < L.nz) {
-            const int c = i + L.nx * (j + L.ny * k);
-            const float ax = gather_lap<DIM>(L, c, i, j, k, [&](int q, int, int, int) { return x[q]; });
+            const uint32_t c = i + L.nx * (j + L.ny * k);
+            const float ax = gather_lap<DIM>(L, c, i, j, k, [&](uint32_t q, int, int, int) { return x[q]; });
             sum += (c == skip ? 0.f : r[c]) - ax;
           }
         }
@@ -144,11 +138,11 @@ template <int DIM, bool PRO>
 __global__ void __launch_bounds__(256) k_resid_g(GLevel G, LV C, const float* __restrict__ x,
                                                  const float* __restrict__ ec, float cw,
                                                  const float* __restrict__ r, float* __restrict__ u,
-                                                 int skip) {
+                                                 uint32_t skip) {
   pdl_enter();
   const LV& L = G.L;
-  gather_cells(G.n, L.nx, L.ny, G.dx, G.dy, [&](int c, int i, int j, int k) {
-    const float ax = gather_lap<DIM>(L, c, i, j, k, [&](int q, int di, int dj, int dk) {
+  gather_cells(G.n, L.nx, L.ny, G.dx, G.dy, [&](uint32_t c, int i, int j, int k) {
+    const float ax = gather_lap<DIM>(L, c, i, j, k, [&](uint32_t q, int di, int dj, int dk) {
       float v = x[q];
       if (PRO) v += cw * ec[gather_parent(C, i + di, j + dj, k + dk)];
       return v;
@@ -161,13 +155,13 @@ __global__ void __launch_bounds__(256) k_resid_g(GLevel G, LV C, const float* __
 template <int DIM, bool HOOK>
 __global__ void __launch_bounds__(256) k_smooth_g(GLevel G, LV C, Kern K, const float* __restrict__ u,
                                                   const float* __restrict__ ec, float cw,
-                                                  float* __restrict__ x, int pin,
+                                                  float* __restrict__ x, uint32_t pin,
                                                   const float* __restrict__ r, Hook hk) {
   pdl_enter();
   const LV& L = G.L;
   double acc[1] = {0.0};
-  gather_cells(G.n, L.nx, L.ny, G.dx, G.dy, [&](int c, int i, int j, int k) {
-    const float s = gather_conv<DIM>(L, K, c, i, j, k, [&](int q) { return u[q]; });
+  gather_cells(G.n, L.nx, L.ny, G.dx, G.dy, [&](uint32_t c, int i, int j, int k) {
+    const float s = gather_conv<DIM>(L, K, c, i, j, k, [&](uint32_t q) { return u[q]; });
     float v = L.isq[c] * s + x[c];
     if (ec) v += cw * ec[gather_parent(C, i, j, k)];
     if (c == pin) v = r[c];
@@ -190,7 +184,7 @@ __global__ void __launch_bounds__(256) k_smooth_g(GLevel G, LV C, Kern K, const 
 
 // p = z - beta p_old, q = A p; p.q, p.r (see k_fcg_dir)
 template <int DIM>
-__global__ void __launch_bounds__(256) k_fcg_dir_g(res::FaceOp<DIM> A, int n, FcgState* S,
+__global__ void __launch_bounds__(256) k_fcg_dir_g(res::FaceOp<DIM> A, uint32_t n, FcgState* S,
                                                    const float* __restrict__ z, double* P0, double* P1,
                                                    double* __restrict__ q, const double* __restrict__ r,
                                                    double* partials, Loop h) {
@@ -201,14 +195,14 @@ __global__ void __launch_bounds__(256) k_fcg_dir_g(res::FaceOp<DIM> A, int n, Fc
   const double beta = first ? 0.0 : S->beta;
   double* __restrict__ pn = (it & 1) ? P1 : P0;
   const double* __restrict__ po = (it & 1) ? P0 : P1;
-  auto val = [&](int c) {
+  auto val = [&](uint32_t c) {
     const double v = (double)z[c];
     return first ? v : fma(-beta, po[c], v);
   };
   double acc[2] = {0.0, 0.0};
   const int sz = (int)A.sz;
-  gather_cells(n, A.nx, A.ny, A.dx, A.dy, [&](int c, int i, int j, int k) {
-    const res::Cf<double> f = A.load((uint32_t)c, i, j, k);
+  gather_cells(n, A.nx, A.ny, A.dx, A.dy, [&](uint32_t c, int i, int j, int k) {
+    const res::Cf<double> f = A.load(c, i, j, k);
     // (couplings across the domain's edge are 0: any value inside will do)
     const double v = val(c);
     const double w = val(i > 0 ? c - 1 : c), e = val(i + 1 < A.nx ? c + 1 : c);

@@ -33,6 +33,7 @@
 #include <cmath>
 #include <cstdint>
 
+#include "cell_index.cuh"
 #include "cfdb.h"
 #include "grid_sync.cuh"
 #include "poperator.cuh"
@@ -40,23 +41,6 @@
 
 namespace cfdb {
 namespace res {
-
-// Division of a cell index (< 2^31) by a fixed divisor: one 32 x 32 -> 64
-// multiply (m = ceil(2^s / d), s = 31 + ceil(log2 d), m < 2^32).
-struct FastDiv {
-  uint32_t m = 0, s = 31;
-  __device__ __forceinline__ uint32_t div(uint32_t c) const {
-    return (uint32_t)(((uint64_t)c * m) >> s);
-  }
-};
-__host__ __device__ inline FastDiv fast_div(uint32_t d) {
-  FastDiv f;
-  uint32_t l = 0;
-  while ((1ull << l) < d) ++l;
-  f.s = 31 + l;
-  f.m = (uint32_t)(((1ull << f.s) + d - 1) / d);
-  return f;
-}
 
 // Couplings of one cell to its neighbours (0 across the domain's edge), its
 // diagonal and the preconditioner's inverse diagonal.

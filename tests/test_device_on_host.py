@@ -163,3 +163,37 @@ int main() {
 """)
     for row, team in zip(LINE, got):
         assert team == ("1" if row[3] < row[4] else "2"), row
+
+
+@pytest.mark.parametrize("n,nx,ny", [(46339 * 46339, 46339, 1), (1290 ** 3, 1290, 1290), (1 << 31, 2, 1 << 20),
+                                     (1000, 10, 10)])
+def test_gathering_passes_end_at_the_last_cell(tmp_path, n, nx, ny):
+    """The one-cell-per-thread loop of the largest grids, as the first and the last thread of a
+    full launch run it: every index below n, the right coordinates, and no step past the end."""
+    got = _run(tmp_path, r"""
+#include "device_on_host.h"
+#include "cell_index.cuh"
+#include <cstdio>
+int main() {
+  const uint32_t n = %du; const int nx = %d, ny = %d;
+  gridDim.x = 2368;
+  for (int last = 0; last < 2; ++last) {
+    blockIdx.x = last ? gridDim.x - 1 : 0;
+    threadIdx.x = last ? 255 : 0;
+    long long count = 0, bad = 0, top = -1;
+    cfdb::res::gather_cells(n, nx, ny, cfdb::res::fast_div(nx), cfdb::res::fast_div(ny),
+                            [&](uint32_t c, int i, int j, int k) {
+      bad += c >= n || i < 0 || i >= nx || j < 0 || j >= ny || k < 0;
+      bad += (uint32_t)(i + (long long)nx * (j + (long long)ny * k)) != c;
+      top = c;
+      if (++count > 10000) { printf("runaway\n"); std::exit(0); }
+    });
+    printf("%%lld %%lld %%lld ", count, top, bad);
+  }
+}
+""" % (n, nx, ny))
+    stride = 2368 * 256
+    for first, (count, top, bad) in zip((0, stride - 1), (map(int, got[:3]), map(int, got[3:]))):
+        want = max(0, -(-(n - first) // stride))
+        assert (count, bad) == (want, 0)
+        assert top == (first + (want - 1) * stride if want else -1)
