@@ -121,8 +121,8 @@ __device__ __forceinline__ void cp_wait() {
   asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
 }
 
-// Thread layout of the tiled kernels: TX x TY threads, each owning CX cells
-// of a plane row strided by TX (so every load instruction is coalesced).
+// Thread layout of the initial residual's tiles: TX x TY threads, one cell of
+// a plane each.
 template <int DIM>
 struct Tile;
 // Shared-memory rows of a plane buffer: the TY rows plus a y-halo row on
@@ -231,9 +231,9 @@ struct Seg {
   int64_t items;
 };
 
-template <int DIM, int CX>
+template <int DIM>
 Seg make_seg(int nx, int ny, int nz) {
-  constexpr int PX = Tile<DIM>::TX * CX, PY = Tile<DIM>::TY;
+  constexpr int PX = Tile<DIM>::TX, PY = Tile<DIM>::TY;
   Seg s;
   s.tiles_x = (nx + PX - 1) / PX;
   const int64_t tiles = (int64_t)s.tiles_x * ((ny + PY - 1) / PY);
@@ -264,68 +264,35 @@ __device__ __forceinline__ void for_runs(const Seg& sg, int nz, F f) {
 }
 
 // 7-point march over planes [k0, k1) of tile (tix, tiy): val(i,j,k) is the
-// stencil input.  For every plane, cell(c, act, i, j, k, v, w, e, s, n, b, t)
-// runs for each of the thread's CX cells, then after(k) runs once in EVERY
-// thread (it may use warp and block collectives).  z-neighbours stay in
-// registers; the plane with its x/y halo is staged in shared memory.
-template <typename T, int TX, int TY, int CX, class Val, class Cell, class After>
+// stencil input.  For every plane, cell(i, j, k, v, w, e, s, n, b, t) runs for
+// the thread's cell if it is in the grid.  z-neighbours stay in registers; the
+// plane with its x/y halo is staged in shared memory.
+template <typename T, int TX, int TY, class Val, class Cell>
 __device__ __forceinline__ void march7(int nx, int ny, int nz, int tix, int tiy, int k0, int k1,
-                                       T (*buf)[Rows<TY>::N][TX * CX + 2], Val val, Cell cell,
-                                       After after) {
-  constexpr int PX = TX * CX, R0 = Rows<TY>::R0;
+                                       T (*buf)[Rows<TY>::N][TX + 2], Val val, Cell cell) {
+  constexpr int R0 = Rows<TY>::R0;
   const int tx = threadIdx.x % TX, ty = threadIdx.x / TX;
-  const int x0 = tix * PX, j = tiy * TY + ty;
-  const bool row = j < ny;
-  T vp[CX], vc[CX], vn[CX];
-#pragma unroll
-  for (int c = 0; c < CX; ++c) {
-    const int i = x0 + tx + c * TX;
-    const bool a = row && i < nx;
-    vp[c] = (a && k0 > 0) ? val(i, j, k0 - 1) : T(0);
-    vc[c] = a ? val(i, j, k0) : T(0);
-  }
+  const int x0 = tix * TX, i = x0 + tx, j = tiy * TY + ty;
+  const bool row = j < ny, act = row && i < nx;
+  T vp = (act && k0 > 0) ? val(i, j, k0 - 1) : T(0);
+  T vc = act ? val(i, j, k0) : T(0);
   for (int k = k0; k < k1; ++k) {
-    T(*s)[PX + 2] = buf[k & 1];
-#pragma unroll
-    for (int c = 0; c < CX; ++c) {
-      const int i = x0 + tx + c * TX;
-      vn[c] = (row && i < nx && k + 1 < nz) ? val(i, j, k + 1) : T(0);
-      s[ty + R0][1 + tx + c * TX] = vc[c];
-    }
+    T(*s)[TX + 2] = buf[k & 1];
+    const T vn = (act && k + 1 < nz) ? val(i, j, k + 1) : T(0);
+    s[ty + R0][1 + tx] = vc;
     if (tx == 0) s[ty + R0][0] = (row && x0 > 0) ? val(x0 - 1, j, k) : T(0);
-    if (tx == TX - 1) s[ty + R0][PX + 1] = (row && x0 + PX < nx) ? val(x0 + PX, j, k) : T(0);
+    if (tx == TX - 1) s[ty + R0][TX + 1] = (row && x0 + TX < nx) ? val(x0 + TX, j, k) : T(0);
     if (TY > 1) {
-      if (ty == 0) {
-#pragma unroll
-        for (int c = 0; c < CX; ++c) {
-          const int i = x0 + tx + c * TX;
-          s[0][1 + tx + c * TX] = (j > 0 && i < nx) ? val(i, j - 1, k) : T(0);
-        }
-      }
-      if (ty == TY - 1) {
-#pragma unroll
-        for (int c = 0; c < CX; ++c) {
-          const int i = x0 + tx + c * TX;
-          s[TY + 1][1 + tx + c * TX] = (j + 1 < ny && i < nx) ? val(i, j + 1, k) : T(0);
-        }
-      }
+      if (ty == 0) s[0][1 + tx] = (j > 0 && i < nx) ? val(i, j - 1, k) : T(0);
+      if (ty == TY - 1) s[TY + 1][1 + tx] = (j + 1 < ny && i < nx) ? val(i, j + 1, k) : T(0);
     }
     __syncthreads();
-#pragma unroll
-    for (int c = 0; c < CX; ++c) {
-      const int xi = 1 + tx + c * TX;
-      const int i = x0 + tx + c * TX;
-      const T vs = (TY > 1) ? s[ty][xi] : T(0);
-      const T vnn = (TY > 1) ? s[ty + 2][xi] : T(0);
-      cell(c, row && i < nx, i, j, k, vc[c], s[ty + R0][xi - 1], s[ty + R0][xi + 1], vs, vnn, vp[c],
-           vn[c]);
+    if (act) {
+      const T south = (TY > 1) ? s[ty][1 + tx] : T(0), north = (TY > 1) ? s[ty + 2][1 + tx] : T(0);
+      cell(i, j, k, vc, s[ty + R0][tx], s[ty + R0][tx + 2], south, north, vp, vn);
     }
-    after(k);
-#pragma unroll
-    for (int c = 0; c < CX; ++c) {
-      vp[c] = vc[c];
-      vc[c] = vn[c];
-    }
+    vp = vc;
+    vc = vn;
   }
   __syncthreads();
 }
@@ -1048,7 +1015,7 @@ void level_res(const MgLevel& M, const LV& LC, const float* x, const float* ec, 
     } else {
       launch(k_resid_g<DIM, false>, g, 256, 0, st, G, LC, x, ec, cw, r, res, (uint32_t)skip);
     }
-  } else if (DIM == 3 && quad_ok<DIM>(M.n[0])) {
+  } else if constexpr (DIM == 3) {
     const Seg sg = make_quad_seg<3>(M.n[0], M.n[1], M.n[2]);
     constexpr int T = PlaneTile::T;
     constexpr size_t SM = res_s_smem();
@@ -1063,17 +1030,17 @@ void level_res(const MgLevel& M, const LV& LC, const float* x, const float* ec, 
       launch(k_res_s<false, false>, quad_wave<3>((const void*)k_res_s<false, false>, sg, SM), T, SM,
              st, L, LC, sg, x, ec, cw, r, res, rc, skip);
   } else {
-    const Seg sg = make_quad_seg<DIM>(M.n[0], M.n[1], M.n[2]);
-    constexpr int T = Quad<DIM>::TX * Quad<DIM>::TY;
+    const Seg sg = make_quad_seg<2>(M.n[0], M.n[1], M.n[2]);
+    constexpr int T = Quad<2>::TX;
     const LV L = lv(M);
     if (rc)
-      launch(k_res_q<DIM, false, true>, quad_wave<DIM>((const void*)k_res_q<DIM, false, true>, sg), T,
+      launch(k_res_q<2, false, true>, quad_wave<2>((const void*)k_res_q<2, false, true>, sg), T,
              0, st, L, LC, sg, x, ec, cw, r, res, rc, skip);
     else if (ec)
-      launch(k_res_q<DIM, true, false>, quad_wave<DIM>((const void*)k_res_q<DIM, true, false>, sg), T,
+      launch(k_res_q<2, true, false>, quad_wave<2>((const void*)k_res_q<2, true, false>, sg), T,
              0, st, L, LC, sg, x, ec, cw, r, res, rc, skip);
     else
-      launch(k_res_q<DIM, false, false>, quad_wave<DIM>((const void*)k_res_q<DIM, false, false>, sg), T,
+      launch(k_res_q<2, false, false>, quad_wave<2>((const void*)k_res_q<2, false, false>, sg), T,
              0, st, L, LC, sg, x, ec, cw, r, res, rc, skip);
   }
 }
@@ -1091,7 +1058,7 @@ void level_sm(const MgLevel& M, const LV& LC, const Kern& K, bool first, const f
       launch(k_smooth_g<DIM, true>, g, 256, 0, st, G, LC, K, src, ec, cw, x, (uint32_t)pin, r, *hook);
     else
       launch(k_smooth_g<DIM, false>, g, 256, 0, st, G, LC, K, src, ec, cw, x, (uint32_t)pin, r, Hook{});
-  } else if (DIM == 3 && quad_ok<DIM>(M.n[0])) {
+  } else if constexpr (DIM == 3) {
     const Seg sg = make_quad_seg<3>(M.n[0], M.n[1], M.n[2]);
     constexpr int T = PlaneTile::T;
     constexpr size_t SM = sm_s_smem();
@@ -1106,17 +1073,17 @@ void level_sm(const MgLevel& M, const LV& LC, const Kern& K, bool first, const f
       launch(k_sm_s<SM_ADD, false>, quad_wave<3>((const void*)k_sm_s<SM_ADD, false>, sg, SM), T, SM,
              st, L, LC, sg, K, src, ec, cw, x, skip, pin, r, Hook{});
   } else {
-    const Seg sg = make_quad_seg<DIM>(M.n[0], M.n[1], M.n[2]);
-    constexpr int T = Quad<DIM>::TX * Quad<DIM>::TY;
+    const Seg sg = make_quad_seg<2>(M.n[0], M.n[1], M.n[2]);
+    constexpr int T = Quad<2>::TX;
     const LV L = lv(M);
     if (first)
-      launch(k_sm_q<DIM, SM_FIRST, false>, quad_wave<DIM>((const void*)k_sm_q<DIM, SM_FIRST, false>, sg),
+      launch(k_sm_q<2, SM_FIRST, false>, quad_wave<2>((const void*)k_sm_q<2, SM_FIRST, false>, sg),
              T, 0, st, L, LC, sg, K, src, ec, cw, x, skip, pin, r, Hook{});
     else if (hook)
-      launch(k_sm_q<DIM, SM_ADD, true>, quad_wave<DIM>((const void*)k_sm_q<DIM, SM_ADD, true>, sg), T, 0,
+      launch(k_sm_q<2, SM_ADD, true>, quad_wave<2>((const void*)k_sm_q<2, SM_ADD, true>, sg), T, 0,
              st, L, LC, sg, K, src, ec, cw, x, skip, pin, r, *hook);
     else
-      launch(k_sm_q<DIM, SM_ADD, false>, quad_wave<DIM>((const void*)k_sm_q<DIM, SM_ADD, false>, sg), T,
+      launch(k_sm_q<2, SM_ADD, false>, quad_wave<2>((const void*)k_sm_q<2, SM_ADD, false>, sg), T,
              0, st, L, LC, sg, K, src, ec, cw, x, skip, pin, r, Hook{});
   }
 }
@@ -1243,31 +1210,28 @@ double cycle_bytes(const MgHierarchy& H, const MgWeights& W) {
 // ------------------------------------------------------------ FCG kernels
 
 // r = b - A x, r32 = float(r); ||r|| decides whether the loop runs at all.
-template <int DIM, int CX>
+template <int DIM>
 __global__ void __launch_bounds__(kT, 2) k_fcg_init(OpView<double> A, Seg sg, FcgState* S,
                                                     double* __restrict__ r, float* __restrict__ r32,
                                                     double* partials, double* hist, int64_t hcap,
                                                     Loop h) {
   pdl_enter();
   constexpr int TX = Tile<DIM>::TX, TY = Tile<DIM>::TY;
-  __shared__ double buf[2][Rows<TY>::N][TX * CX + 2];
+  __shared__ double buf[2][Rows<TY>::N][TX + 2];
   const double* __restrict__ b = S->b;
   const double* __restrict__ x = S->x;
   double acc[1] = {0.0};
   auto val = [&](int i, int j, int k) { return x[i + (int64_t)A.nx * (j + (int64_t)A.ny * k)]; };
   for_runs(sg, A.nz, [&](int tix, int tiy, int k0, int k1) {
-    march7<double, TX, TY, CX>(
+    march7<double, TX, TY>(
         A.nx, A.ny, A.nz, tix, tiy, k0, k1, buf, val,
-        [&](int, bool act, int i, int j, int k, double v, double w, double e, double s, double n,
-            double bo, double t) {
-          if (!act) return;
+        [&](int i, int j, int k, double v, double w, double e, double s, double n, double bo, double t) {
           const int64_t c = i + (int64_t)A.nx * (j + (int64_t)A.ny * k);
           const double rn = b[c] - apply_coef(load_coef(A, i, j, k), v, w, e, s, n, bo, t);
           r[c] = rn;
           r32[c] = (float)rn;
           acc[0] += rn * rn;
-        },
-        [](int) {});
+        });
   });
   reduce_last<1>(acc, partials, &S->ticket, [&](const double* tot) {
     const double b0 = sqrt(tot[0]);
@@ -1540,10 +1504,10 @@ namespace {
 // 2D quad passes run up to 32 blocks of 64 threads per SM.
 int64_t partial_slots(const FineOperator&) { return std::max(kMaxBlocks, 148 * 32); }
 
-template <int DIM, int CX>
+template <int DIM>
 void launch_init_t(LearnedSolver* s, const FineOperator& op, Loop h, cudaStream_t st) {
-  const Seg sg = make_seg<DIM, CX>(op.A.nx, op.A.ny, op.A.nz);
-  launch(k_fcg_init<DIM, CX>, seg_grid(sg), kT, 0, st, op.A, sg, s->S, s->r, s->r32, s->partials,
+  const Seg sg = make_seg<DIM>(op.A.nx, op.A.ny, op.A.nz);
+  launch(k_fcg_init<DIM>, seg_grid(sg), kT, 0, st, op.A, sg, s->S, s->r, s->r32, s->partials,
          s->hist, s->hist_cap, h);
 }
 
@@ -1555,30 +1519,20 @@ void launch_dir_g(LearnedSolver* s, const FineOperator& op, Loop h, cudaStream_t
 }
 
 void launch_init(LearnedSolver* s, const FineOperator& op, Loop h, cudaStream_t st) {
-  if (op.dim == 2) launch_init_t<2, 1>(s, op, h, st);
-  else launch_init_t<3, 1>(s, op, h, st);
+  if (op.dim == 2) launch_init_t<2>(s, op, h, st);
+  else launch_init_t<3>(s, op, h, st);
 }
 
-template <int DIM>
-[[maybe_unused]] void launch_dir_v(LearnedSolver* s, const FineOperator& op, Loop h, cudaStream_t st) {
-  const int64_t nq = (int64_t)(op.A.nx / 4) * op.A.ny * op.A.nz;
-  const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((nq + 255) / 256, kGridCap));
-  launch(k_fcg_dir_v<DIM>, grid, 256, 0, st, op.A, s->S, s->z32, s->p0, s->p1, s->q, s->r,
-         s->partials, h);
-}
-
-template <int DIM>
 void launch_dir_q(LearnedSolver* s, const FineOperator& op, Loop h, cudaStream_t st) {
-  const Seg sg = make_quad_seg<DIM>(op.A.nx, op.A.ny, op.A.nz);
-  if (!op.A.fx && !op.A.fy && !op.A.fz) {
-    const int grid = quad_grid<DIM>(sg, (int64_t)dir_blocks_per_sm<DIM, true>() * 148);
-    launch(k_fcg_dir_q<DIM, true>, grid, Quad<DIM>::TX * Quad<DIM>::TY, 0, st, op.A, sg, s->S,
-           s->z32, s->p0, s->p1, s->q, s->r, s->partials, h);
-    return;
-  }
-  const int grid = quad_grid<DIM>(sg, (int64_t)dir_blocks_per_sm<DIM>() * 148);
-  launch(k_fcg_dir_q<DIM>, grid, Quad<DIM>::TX * Quad<DIM>::TY, 0, st, op.A, sg, s->S, s->z32,
-         s->p0, s->p1, s->q, s->r, s->partials, h);
+  const Seg sg = make_quad_seg<2>(op.A.nx, op.A.ny, op.A.nz);
+  const bool tables = !op.A.fx && !op.A.fy && !op.A.fz;
+  const int grid = quad_grid<2>(sg, (int64_t)dir_blocks_per_sm(tables) * 148);
+  if (tables)
+    launch(k_fcg_dir_q<2, true>, grid, Quad<2>::TX, 0, st, op.A, sg, s->S, s->z32, s->p0, s->p1, s->q,
+           s->r, s->partials, h);
+  else
+    launch(k_fcg_dir_q<2, false>, grid, Quad<2>::TX, 0, st, op.A, sg, s->S, s->z32, s->p0, s->p1, s->q,
+           s->r, s->partials, h);
 }
 
 void launch_dir_s(LearnedSolver* s, const FineOperator& op, Loop h, cudaStream_t st) {
@@ -1592,12 +1546,12 @@ void launch_dir_s(LearnedSolver* s, const FineOperator& op, Loop h, cudaStream_t
     launch(k_dir_s<false>, quad_wave<3>((const void*)k_dir_s<false>, sg, SM), PlaneTile::T, SM, st,
            op.A, sg, s->S, s->z32, s->p0, s->p1, s->q, s->r, s->partials, h);
   else
-    launch_dir_v<3>(s, op, h, st);
+    launch_dir_g<3>(s, op, h, st);
 }
 
 void launch_dir(LearnedSolver* s, const FineOperator& op, Loop h, cudaStream_t st) {
   if (op.dim == 2) {
-    if (quad_ok<2>(op.A.nx) && s->cells > kGatherDirCells) launch_dir_q<2>(s, op, h, st);
+    if (quad_ok<2>(op.A.nx) && s->cells > kGatherDirCells) launch_dir_q(s, op, h, st);
     else launch_dir_g<2>(s, op, h, st);
   } else {
     // 3D: the staged pass

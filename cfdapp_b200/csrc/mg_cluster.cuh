@@ -349,7 +349,7 @@ struct FcgArgs {
 };
 
 // A whole FCG(1) solve of a small system: k_fcg_init, the V-cycle,
-// k_fcg_dir and k_fcg_update of the graph form, with its stopping tests.
+// direction pass and k_fcg_update of the graph form, with its stopping tests.
 // p keeps halo planes that its readers update themselves from the pushed z.
 template <int DIM>
 __global__ void __launch_bounds__(kClusterT, 1)

@@ -151,7 +151,7 @@ __global__ void __launch_bounds__(256) k_resid_g(GLevel G, LV C, const float* __
   });
 }
 
-// x += [cw P ec] + D^-1/2 (W * u); pin >= 0: x[pin] = r[pin]; HOOK: z.q (see k_sm)
+// x += [cw P ec] + D^-1/2 (W * u); pin >= 0: x[pin] = r[pin]; HOOK: z.q
 template <int DIM, bool HOOK>
 __global__ void __launch_bounds__(256) k_smooth_g(GLevel G, LV C, Kern K, const float* __restrict__ u,
                                                   const float* __restrict__ ec, float cw,
@@ -182,7 +182,7 @@ __global__ void __launch_bounds__(256) k_smooth_g(GLevel G, LV C, Kern K, const 
   }
 }
 
-// p = z - beta p_old, q = A p; p.q, p.r (see k_fcg_dir)
+// p = z - beta p_old (p = z on the first iteration), q = A p; p.q, p.r
 template <int DIM>
 __global__ void __launch_bounds__(256) k_fcg_dir_g(res::FaceOp<DIM> A, uint32_t n, FcgState* S,
                                                    const float* __restrict__ z, double* P0, double* P1,

@@ -4,7 +4,11 @@
 // vectors and the stencil reads a thread's own x-neighbours from registers
 // and its own shared-memory row.  Used where the row length is a multiple of
 // 4 and at least one tile wide and the level is large; the one-cell-per-thread
-// kernels of mg_gather.cuh cover every other level.
+// kernels of mg_gather.cuh cover every other level.  The kernels here are
+// launched in 2D; 3D levels take the staged ones (mg_stage.cuh), which share
+// the tile and the vector helpers.  (The kernels stay written over DIM: with
+// the y terms, zeros in 2D, dropped, a 2048^2 FCG iteration took 245 us
+// against 239.)
 //
 // Tile: TX x TY threads own a (4*TX) x TY patch of an (x,y) plane and march
 // along z through a run of planes that starts on an even one (a coarse
@@ -146,11 +150,10 @@ __device__ __forceinline__ void coef4(const LV& L, int i0, int j, int k, float (
   zh = ld4(L.fz + c + (int64_t)L.nx * L.ny);
 }
 
-// The quad counterpart of k_res (see there).
-// 3D: four resident blocks per SM (64 registers, no spills): 2.6 % faster
-// per FCG iteration at 256^3; 2D keeps the compiler's own allocation.
+// res = r - A x  (PRO: x + cw P ec in place of x).  RESTRICT: instead of
+// storing res, rc(parent) = sum of the children's res.  r[skip] reads as 0.
 template <int DIM, bool PRO, bool RESTRICT>
-__global__ void __launch_bounds__(Quad<DIM>::TX* Quad<DIM>::TY, DIM == 3 ? 4 : 0)
+__global__ void __launch_bounds__(Quad<DIM>::TX* Quad<DIM>::TY)
     k_res_q(LV L, LV C, Seg sg, const float* __restrict__ x, const float* __restrict__ ec, float cw,
             const float* __restrict__ r, float* __restrict__ res, float* __restrict__ rc,
             int64_t skip) {
@@ -232,8 +235,11 @@ __global__ void __launch_bounds__(Quad<DIM>::TX* Quad<DIM>::TY, DIM == 3 ? 4 : 0
   });
 }
 
-// The quad counterpart of k_sm (see there): 27-point (2D: 9-point)
-// convolution over a three-plane ring of staged rows.
+// x <- [x] (+ cw P ec) + D^-1/2 (W * (D^-1/2 u)), u = res (SM_ADD) or r with
+// r[skip] = 0 and x = 0 before (SM_FIRST): the 27-point (2D: 9-point)
+// convolution over a ring of three staged planes.  pin >= 0: x[pin] = r[pin]
+// (the last sweep of level 0); HOOK: also accumulates z.q for the FCG
+// coefficient.
 template <int DIM, int MODE, bool HOOK>
 __global__ void __launch_bounds__(Quad<DIM>::TX* Quad<DIM>::TY)
     k_sm_q(LV L, LV C, Seg sg, Kern K, const float* __restrict__ src, const float* __restrict__ ec,
@@ -340,7 +346,7 @@ __global__ void __launch_bounds__(Quad<DIM>::TX* Quad<DIM>::TY)
   });
   if (HOOK) {
     double acc[1] = {acc_dot};
-    reduce_last<1, DIM == 3>(acc, hk.partials, &hk.S->ticket, [&](const double* tot) {
+    reduce_last<1, false>(acc, hk.partials, &hk.S->ticket, [&](const double* tot) {
       FcgState* S = hk.S;
       if (S->it == 0) return;  // the first direction is z itself
       const double beta = tot[0] / S->pq;
@@ -353,18 +359,16 @@ __global__ void __launch_bounds__(Quad<DIM>::TX* Quad<DIM>::TY)
   }
 }
 
-// The quad counterpart of the FCG direction pass (see k_fcg_dir).
+// p = z - beta p_old (p = z on the first iteration), q = A p, and the dot
+// products p.q and p.r that give alpha.
 // Resident blocks per SM of the direction pass (its register budget); its
 // grid is one wave of them, so every block marches a long run of planes.
 // TABLES: the operator's couplings are its per-axis tables (a uniform
 // operator), which needs fewer registers than the per-face form.
-template <int DIM, bool TABLES = false>
-constexpr int dir_blocks_per_sm() {
-  return DIM == 3 ? 2 : (TABLES ? 12 : 8);
-}
+constexpr int dir_blocks_per_sm(bool tables) { return tables ? 12 : 8; }
 
-template <int DIM, bool TABLES = false>
-__global__ void __launch_bounds__(Quad<DIM>::TX* Quad<DIM>::TY, dir_blocks_per_sm<DIM, TABLES>())
+template <int DIM, bool TABLES>
+__global__ void __launch_bounds__(Quad<DIM>::TX* Quad<DIM>::TY, dir_blocks_per_sm(TABLES))
     k_fcg_dir_q(OpView<double> A, Seg sg, FcgState* S, const float* __restrict__ z, double* P0,
                 double* P1, double* __restrict__ q, const double* __restrict__ r, double* partials,
                 Loop h) {
@@ -458,120 +462,7 @@ __global__ void __launch_bounds__(Quad<DIM>::TX* Quad<DIM>::TY, dir_blocks_per_s
         },
         [](int) {});
   });
-  reduce_last<2, DIM == 3>(acc, partials, &S->ticket, [&](const double* tot) {
-    const double pq = tot[0], pr = tot[1];
-    const double alpha = pr / pq;
-    if (!isfinite(pq) || !(pq > 0.0) || !isfinite(alpha)) {
-      stop_loop(S, h, kLearnedStagnated);
-      return;
-    }
-    S->pq = pq;
-    S->pr = pr;
-    S->alpha = alpha;
-  });
-}
-
-// The direction pass without a marching tile: one thread per four-cell quad,
-// its six neighbour values read straight from global memory (L1/L2 serve the
-// re-reads of the neighbouring quads), so a thread keeps little state and
-// many warps stay resident to hide DRAM latency.  Same arithmetic and
-// coefficient order as k_fcg_dir_q.
-template <int DIM>
-__global__ void __launch_bounds__(256) k_fcg_dir_v(OpView<double> A, FcgState* S,
-                                                   const float* __restrict__ z, double* P0,
-                                                   double* P1, double* __restrict__ q,
-                                                   const double* __restrict__ r, double* partials,
-                                                   Loop h) {
-  pdl_enter();
-  if (S->done) return;
-  const long long it = S->it;
-  const bool first = (it == 0);
-  const double beta = first ? 0.0 : S->beta;
-  double* __restrict__ pn = (it & 1) ? P1 : P0;
-  const double* __restrict__ po = (it & 1) ? P0 : P1;
-  const int nx = A.nx, ny = A.ny, nz = A.nz, qxn = nx >> 2;
-  const int nq = qxn * ny * nz;
-  const int64_t plane = (int64_t)nx * ny;
-  auto val4 = [&](int64_t c) {
-    const V4<float> zz = ld4(z + c);
-    V4<double> v;
-    if (first) {
-#pragma unroll
-      for (int t = 0; t < 4; ++t) v.v[t] = (double)zz.v[t];
-    } else {
-      const V4<double> p = ld4(po + c);
-#pragma unroll
-      for (int t = 0; t < 4; ++t) v.v[t] = fma(-beta, p.v[t], (double)zz.v[t]);
-    }
-    return v;
-  };
-  auto val1 = [&](int64_t c) { return first ? (double)z[c] : fma(-beta, po[c], (double)z[c]); };
-  const V4<double> zero{{0.0, 0.0, 0.0, 0.0}};
-  double acc[2] = {0.0, 0.0};
-  for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < nq; g += gridDim.x * blockDim.x) {
-    const int qx = g % qxn, rest = g / qxn;
-    const int j = rest % ny, k = rest / ny;
-    const int i0 = 4 * qx;
-    const int64_t c = i0 + (int64_t)nx * (j + (int64_t)ny * k);
-    const V4<double> v = val4(c);
-    const double wl = i0 > 0 ? val1(c - 1) : 0.0;
-    const double er = i0 + 4 < nx ? val1(c + 4) : 0.0;
-    const V4<double> s = (DIM == 3 && j > 0) ? val4(c - nx) : zero;
-    const V4<double> n = (DIM == 3 && j + 1 < ny) ? val4(c + nx) : zero;
-    const V4<double> b = k > 0 ? val4(c - plane) : zero;
-    const V4<double> t = k + 1 < nz ? val4(c + plane) : zero;
-    double fx[5];
-    if (A.fx) {
-      const int64_t bx = i0 + (int64_t)(nx + 1) * (j + (int64_t)ny * k);
-#pragma unroll
-      for (int u = 0; u < 5; ++u) fx[u] = A.fx[bx + u];
-    } else {
-#pragma unroll
-      for (int u = 0; u < 5; ++u) fx[u] = A.tx[i0 + u];
-    }
-    V4<double> yl, yh, zl, zh;
-    if (A.fy) {
-      const int64_t by = i0 + (int64_t)nx * (j + (int64_t)(ny + 1) * k);
-      yl = ld4(A.fy + by);
-      yh = ld4(A.fy + by + nx);
-    } else {
-      const double a = A.ty[j], bb = A.ty[j + 1];
-      yl = V4<double>{{a, a, a, a}};
-      yh = V4<double>{{bb, bb, bb, bb}};
-    }
-    if (A.fz) {
-      zl = ld4(A.fz + c);
-      zh = ld4(A.fz + c + plane);
-    } else {
-      const double a = A.tz[k], bb = A.tz[k + 1];
-      zl = V4<double>{{a, a, a, a}};
-      zh = V4<double>{{bb, bb, bb, bb}};
-    }
-    V4<double> aq;
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const double w = u == 0 ? wl : v.v[u - 1];
-      const double e = u == 3 ? er : v.v[u + 1];
-      // diagonal summed in the reference's face order (as load_coef)
-      const double d = ((((fx[u] + fx[u + 1]) + yl.v[u]) + yh.v[u]) + zl.v[u]) + zh.v[u];
-      double off = fx[u] * w;
-      off = fma(fx[u + 1], e, off);
-      off = fma(yl.v[u], s.v[u], off);
-      off = fma(yh.v[u], n.v[u], off);
-      off = fma(zl.v[u], b.v[u], off);
-      off = fma(zh.v[u], t.v[u], off);
-      aq.v[u] = (A.pinned && c + u == A.ref) ? v.v[u] : fma(d, v.v[u], -off);
-    }
-    st4(pn + c, v);
-    st4(q + c, aq);
-    const V4<double> rr = ld4(r + c);
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      acc[0] += v.v[u] * aq.v[u];
-      acc[1] += v.v[u] * rr.v[u];
-    }
-  }
-  reduce_last<2>(acc, partials, &S->ticket, [&](const double* tot) {
+  reduce_last<2, false>(acc, partials, &S->ticket, [&](const double* tot) {
     const double pq = tot[0], pr = tot[1];
     const double alpha = pr / pq;
     if (!isfinite(pq) || !(pq > 0.0) || !isfinite(alpha)) {

@@ -1,6 +1,6 @@
 // Staged variants of the 3D wide-level FCG and V-cycle passes (included by
 // mg.cu inside its anonymous namespace, after mg_quad.cuh): the same
-// per-cell arithmetic as k_res_q / k_sm_q / k_fcg_dir_v, with every plane
+// per-cell arithmetic as the 2D k_res_q / k_sm_q / k_fcg_dir_q, with every plane
 // tile brought into shared memory by cp.async D planes ahead of its use, so
 // a block keeps loads in flight while it computes instead of stalling on
 // each plane's halo and couplings.  Measured on the B200 at 256^3 (warm, per

@@ -719,8 +719,7 @@ bool on_chip(const cfdb_context* ctx, const cfdb_poperator* op, size_t word) {
 
 // Plain FP64 PCG on device vectors.
 cfdb_status solve_fp64(cfdb_context* ctx, cfdb_poperator* op, const cfdb_linear_settings* s,
-                       const double* b, double* x, bool x0_zero, int64_t hist_cap,
-                       cfdb_linear_result* res) {
+                       const double* b, double* x, int64_t hist_cap, cfdb_linear_result* res) {
   const int64_t n = op->cells;
   // on chip where it fits: the exchanged values (w64[1]) and the inverse
   // diagonal of a table operator (w64[6]) are its only vectors in memory
@@ -737,7 +736,7 @@ cfdb_status solve_fp64(cfdb_context* ctx, cfdb_poperator* op, const cfdb_linear_
                       op->invd64 ? nullptr : op->w64[6],
                       ResidentLimits{s->abs_tol, s->rel_tol, s->max_iterations, op->hist_dev, hist_cap, 0.0, 0});
   else
-    st = run_pcg<double>(ctx, op, b, x, op->w64[0], op->w64[1], op->w64[2], op->w64[6], x0_zero ? 1 : 0,
+    st = run_pcg<double>(ctx, op, b, x, op->w64[0], op->w64[1], op->w64[2], op->w64[6], 0,
                          s->abs_tol, s->rel_tol, s->max_iterations, op->hist_dev, hist_cap);
   if (st != CFDB_OK) return st;
   st = read_scalars(ctx, 8);
@@ -747,7 +746,7 @@ cfdb_status solve_fp64(cfdb_context* ctx, cfdb_poperator* op, const cfdb_linear_
   res->iterations = (int64_t)o[OUT_ITER];
   res->initial_residual = o[OUT_B0];
   res->final_residual = o[OUT_FINAL];
-  res->krylov_bytes += pcg_bytes(op, sizeof(double), res->iterations, x0_zero);
+  res->krylov_bytes += pcg_bytes(op, sizeof(double), res->iterations, false);
   return add_krylov_time(ctx, res);
 }
 
@@ -951,7 +950,7 @@ cfdb_status solve_learned(cfdb_context* ctx, cfdb_poperator* op, const cfdb_line
     s2.rel_tol = s->rel_tol * res->initial_residual / o.final_residual;
   cfdb_linear_result sub;
   std::memset(&sub, 0, sizeof(sub));
-  st = solve_fp64(ctx, op, &s2, b, x, false, 0, &sub);
+  st = solve_fp64(ctx, op, &s2, b, x, 0, &sub);
   if (st != CFDB_OK) return st;
   res->status = sub.status;
   res->iterations += sub.iterations;
@@ -1300,7 +1299,7 @@ cfdb_status cfdb_poperator_solve_device(cfdb_context* ctx, const cfdb_poperator*
   } else if (s->precision == CFDB_PRECISION_FP32_REFINED) {
     st = solve_refined(ctx, op, s, b_dev, x_dev, history_cap, history, result);
   } else {
-    st = solve_fp64(ctx, op, s, b_dev, x_dev, false, history_cap, result);
+    st = solve_fp64(ctx, op, s, b_dev, x_dev, history_cap, result);
     if (st == CFDB_OK && history && history_cap > 0) {
       const int64_t m = std::min<int64_t>(history_cap, result->iterations + 1);
       CFDB_CUDA(ctx, cudaMemcpyAsync(history, op->hist_dev, sizeof(double) * m,
