@@ -325,3 +325,25 @@ def test_batch_clusters_with_empty_blocks(ctx, method):
     for k, case in enumerate(cases):
         _check_against_single(ctx, case, st, b.get_state(k), res[k], bar=1e-8)
     b.close()
+
+
+@pytest.mark.parametrize("method", ["cg", "bicgstab"])
+def test_batch_of_many_cases_through_teams(ctx, method):
+    """64 cases of 10^2 to 17^2, too many for clusters to pay: both solve stages go through block
+    teams.  Every eighth case against the single-case session (linear solves to 1e-12; 1e-8 as
+    above)."""
+    from cfdapp_b200.cfdb import Batch, LinearSolverSettings, SIMPLESettings, SimpleCase
+    ps = LinearSolverSettings(type=method, preconditioner="jacobi", absolute_tolerance=0.0,
+                              relative_tolerance=1e-12, max_iterations=2000)
+    ms = LinearSolverSettings(type="bicgstab", preconditioner="none", absolute_tolerance=0.0,
+                              relative_tolerance=1e-12, max_iterations=500)
+    st = SIMPLESettings(max_iterations=3, momentum_solver=ms, pressure_solver=ps)
+    cases = [SimpleCase.cavity(2, 10 + (k // 8), mu=0.01 * (1 + k % 3)) for k in range(64)]
+    b = Batch(ctx, cases, st)
+    for k in range(64):
+        b.set_state(k)
+    b.iterate(3)
+    res = b.results()
+    for k in range(0, 64, 8):
+        _check_against_single(ctx, cases[k], st, b.get_state(k), res[k], bar=1e-8)
+    b.close()

@@ -1,6 +1,7 @@
 """Device routines that a host compiler takes (device_on_host.h), run on the CPU
 with a team of one block and one thread that records what the team is asked to do.
 """
+import math
 import os
 import subprocess
 
@@ -197,3 +198,43 @@ int main() {
         want = max(0, -(-(n - first) // stride))
         assert (count, bad) == (want, 0)
         assert top == (first + (want - 1) * stride if want else -1)
+
+
+# the plans behind the grids of test_large_gpu.py on 148 SMs: system, bytes of a word, method
+# (0 CG, 1 BiCGSTAB) -> team, most cells a thread, x and the neighbouring planes on chip
+PLANS = [((787, 773), 8, 0, (2, 5, 1, 1)), ((89, 83, 84), 8, 0, (2, 5, 1, 1)),
+         ((1123, 1117), 8, 0, (2, 9, 1, 1)), ((109, 107, 105), 8, 0, (2, 9, 1, 0)),
+         ((1231, 1229), 8, 0, (2, 10, 0, 1)), ((115, 115, 115), 8, 0, (2, 11, 0, 0)),
+         ((128, 128, 128), 8, 0, (2, 14, 0, 0)), ((1460, 1456), 8, 0, None), ((1459, 1457), 8, 0, None),
+         ((132, 128, 126), 8, 0, None), ((131, 129, 127), 8, 0, None),
+         ((640, 500), 8, 0, (2, 3, 1, 1)), ((128, 128, 32), 8, 0, (2, 4, 1, 0)),
+         ((128, 116, 104), 8, 0, (2, 11, 0, 0)), ((203, 201), 4, 0, (2, 1, 1, 1)),
+         ((45, 43, 41), 4, 0, (2, 2, 1, 1)), ((703, 433), 4, 0, (2, 3, 1, 1)),
+         ((181, 161, 11), 4, 0, (2, 3, 1, 0)), ((125, 121, 119), 4, 0, (2, 12, 0, 1)),
+         ((1459, 1457), 4, 0, None), ((131, 129, 127), 4, 0, None),
+         ((887, 853), 8, 1, (2, 10, 0, 0)), ((93, 91, 89), 8, 1, (2, 10, 0, 0)),
+         ((951, 901), 8, 1, None), ((97, 95, 93), 8, 1, None)]
+
+
+def test_plans_of_large_systems(tmp_path):
+    rows = "".join("{%d,%d,%d,%d}," % (int(math.prod(n)), n[0] if len(n) == 2 else n[0] * n[1],
+                                       word, krylov) for n, word, krylov, _ in PLANS)
+    got = _run(tmp_path, r"""
+#include "device_on_host.h"
+#include "resident_launch.cuh"
+#include <cstdio>
+using namespace cfdb::res;
+int main() {
+  const int rows[][4] = {""" + rows + r"""};
+  for (auto& r : rows) {
+    const Plan P = r[3] == 1 ? bicgstab_plan(r[0], 148, 0) : cg_plan(r[0], r[1], 148, 0, r[2]);
+    printf("%d %d %d %d ", P.team, P.nc, (int)P.xs, (int)P.halo);
+  }
+}
+""")
+    got = [tuple(map(int, got[4 * q:4 * q + 4])) for q in range(len(PLANS))]
+    for row, g in zip(PLANS, got):
+        if row[3] is None:
+            assert g[0] == 0, (row, g)
+        else:
+            assert g == row[3], (row, g)
