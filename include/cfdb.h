@@ -114,7 +114,11 @@ typedef struct {
   double device_ms;           /* device time of the solve (CUDA events, launching stream) */
   int64_t kernel_launches;    /* kernels this library launched for the solve */
   double krylov_ms;           /* device time inside the persistent Krylov kernels */
-  double krylov_bytes;        /* algorithmic bytes those kernels move (words read + written) */
+  double krylov_bytes;        /* algorithmic bytes of those kernels' sweeps: the words of the
+                                 method's vectors and couplings that they read and write, each
+                                 once a sweep, as the kernels for large systems move them.  A
+                                 small system's vectors stay on chip: the figure is then the
+                                 work done, not traffic */
   int64_t krylov_launches;    /* number of persistent Krylov kernel launches */
   int64_t fallback_iterations;/* LEARNED_MG: Jacobi-PCG iterations after a stagnated learned solve */
 } cfdb_linear_result;
