@@ -22,8 +22,12 @@ LIB = os.path.join(LIBDIR, "libcfdb.so")
 OBJDIR = os.path.join(PKG, "_build")
 
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
-NVCC_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "--expt-relaxed-constexpr", "--extended-lambda",
-              "-Xcompiler", "-fPIC", "-Xcompiler", "-O2", "-Xcompiler", "-fvisibility=hidden"]
+# Device code is stored as it is: the driver unpacks a compressed module on its
+# first use (a process's first mixed-precision solve of 128^2 11 ms instead of
+# 16.5, of 96x80x64 21 instead of 29), and nvcc compresses the larger ones.
+NVCC_FLAGS = ["-O3", "--compress-mode=none", "-std=c++17", "-lineinfo",
+              "--expt-relaxed-constexpr", "--extended-lambda", "-Xcompiler", "-fPIC",
+              "-Xcompiler", "-O2", "-Xcompiler", "-fvisibility=hidden"]
 # The SIMPLE stage kernels restate the reference's arithmetic operation by
 # operation; they are compiled without FMA contraction so that a stage
 # reproduces the reference bit for bit (the solvers keep FMA); the batched

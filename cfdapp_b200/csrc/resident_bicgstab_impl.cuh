@@ -53,8 +53,9 @@ cudaError_t launch_bicgstab(cfdb_context* ctx, const BandOp<DIM>& A, const Plan&
     });
   return with_cells(P.nc, [&](auto nc) {
     constexpr int NC = decltype(nc)::value;
-    const void* fn = P.xs ? (const void*)bicgstab_grid<DIM, NC, PREC, true>
-                          : (const void*)bicgstab_grid<DIM, NC, PREC, false>;
+    const void* fn = (const void*)bicgstab_grid<DIM, NC, PREC, true>;
+    if constexpr (NC == 0)  // x of one or two cells a thread always fits
+      if (!P.xs) fn = (const void*)bicgstab_grid<DIM, NC, PREC, false>;
     return cooperative<DIM>(fn, P, ctx->stream, A, n, w, io);
   });
 }

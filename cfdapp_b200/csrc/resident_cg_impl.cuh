@@ -51,9 +51,10 @@ cudaError_t launch_cg(cfdb_context* ctx, const BandOp<DIM>& A, const Plan& P, ui
     const void* fn = P.halo ? (const void*)cg_grid<DIM, T, NC, true, true>
                             : (const void*)cg_grid<DIM, T, NC, true, false>;
     if constexpr (T == kGridThreadsLarge) {  // a small block's x always fits (cg_plan)
-      if (!P.xs)
-        fn = P.halo ? (const void*)cg_grid<DIM, T, NC, false, true>
-                    : (const void*)cg_grid<DIM, T, NC, false, false>;
+      if (!P.xs && P.halo) fn = (const void*)cg_grid<DIM, T, NC, false, true>;
+      // alone, p, r and x leave the block's memory only at the most cells a thread
+      if constexpr ((size_t)3 * NC * T * sizeof(double) > kSmemMax)
+        if (!P.xs && !P.halo) fn = (const void*)cg_grid<DIM, T, NC, false, false>;
     }
     return cooperative<DIM>(fn, P, ctx->stream, A, n, w, io);
   };

@@ -1,7 +1,7 @@
 // Launch of the on-chip Jacobi-PCG (resident_faces.cu), instantiated for one
 // dimension and kind per translation unit: a process loads only the modules
-// it runs.  With every variant in one module the driver took 70 ms to unpack
-// it at a process's first solve; one of these takes 3-15 ms.
+// it runs.  With every variant in one module a process's first solve took
+// 70 ms longer; with one of these it takes 5-9 ms longer than the next.
 #pragma once
 
 #include <cuda_runtime.h>

@@ -60,9 +60,10 @@ cfdb_status pcg_on_chip(cfdb_context* ctx, const OpView<Value<KIND>>& V, const V
       const void* fn = P.halo ? (const void*)pcg_grid<DIM, T, NC, true, true, KIND>
                               : (const void*)pcg_grid<DIM, T, NC, true, false, KIND>;
       if constexpr (T == kGridThreadsLarge) {  // a small block's x always fits (cg_plan)
-        if (!P.xs)
-          fn = P.halo ? (const void*)pcg_grid<DIM, T, NC, false, true, KIND>
-                      : (const void*)pcg_grid<DIM, T, NC, false, false, KIND>;
+        if (!P.xs && P.halo) fn = (const void*)pcg_grid<DIM, T, NC, false, true, KIND>;
+        // alone, p, r and x leave the block's memory only at the most cells a thread
+        if constexpr ((size_t)3 * NC * T * sizeof(Value<KIND>) > kSmemMax)
+          if (!P.xs && !P.halo) fn = (const void*)pcg_grid<DIM, T, NC, false, false, KIND>;
       }
       cudaError_t q = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMax);
       if (q != cudaSuccess) return q;
