@@ -282,7 +282,7 @@ __global__ void __launch_bounds__(krylov::kThreads, 5) k_batch_krylov(KArgs A) {
 // cluster: a cluster of 16 blocks per case, on chip (resident.cuh).  Seven
 // clusters run at once (112 SMs); the others start as these finish, heaviest
 // case first.  An outer iteration of 12 cavities and channels of 48^2 to
-// 256^2 with FP64 CG takes 26.6 ms, against 51.6 ms with teams.
+// 256^2 with FP64 CG takes 25 to 27 ms, against 51 to 53 ms with teams.
 template <int DIM, int NC, int KRYLOV, bool PREC>
 __global__ void __launch_bounds__(res::kClusterThreads, 1) k_batch_cluster(KArgs A) {
   extern __shared__ __align__(16) double sm[];

@@ -503,9 +503,8 @@ __device__ __forceinline__ float coarse_conv(const CoarseGeo<DIM>& G, const Kern
 // the grid kernels; the first smoothing's scaled residual isq r is formed
 // once per cell instead of once per tap, x and res carry a zero halo, and
 // all indexing is 32-bit: the kernel runs on one SM and is bound by its
-// instruction issue.  Cell coordinates come from a float reciprocal (exact
-// below 2^22 cells); the coarsest level's damped-Jacobi sweeps run on only
-// the warps that own its cells (a named barrier instead of the whole block).
+// instruction issue.  Cell coordinates come from FastDiv; every level is worked
+// on by only the warps that own its cells (coarse_cycle).
 
 // Zeroes the padded vectors (their halos stay zero).
 template <int DIM>

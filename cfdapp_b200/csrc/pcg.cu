@@ -13,11 +13,11 @@
 // the device with no host round trip (the reference synchronises and sums on
 // the host once per reduction, DeviceVectorOpsKernel.cu:226-260).
 //
-// Systems that fit the chip's shared memory (up to 128^3) take the on-chip
-// form of the same method instead (resident.cuh); the streaming kernels here
-// serve the larger ones and the FP32-refined solves.
+// Systems that fit the chip's shared memory (about 2.1 M cells: up to 128^3)
+// take the on-chip form of the same method instead (resident.cuh), in FP64,
+// mixed precision and FP32; the streaming kernels here serve the larger ones.
 //
-// The FP32-refined method runs the same kernel in FP32 (FP64 reductions)
+// The FP32-refined method runs the same method in FP32 (FP64 reductions)
 // inside FP64 iterative refinement: r = b - A x in FP64 (fused with the update
 // x += e), inner PCG on A e = r in FP32 to a moderate reduction, repeat until
 // the FP64 true residual meets the tolerance.
