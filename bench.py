@@ -188,8 +188,8 @@ NCU_TRAFFIC = {"batched_pprime_dram_bytes_per_launch": 521465025024.0}
 # DRAM bytes of the learned-FCG solve graph of each benchmark system: its start
 # kernel plus one FCG iteration (learned_fcg_dram_traffic.md); a solve's
 # traffic is start + iterations x per_iteration.
-LEARNED_TRAFFIC = {(2, 2048): {"start": 0.08e9, "per_iteration": 0.6188e9},
-                   (3, 256): {"start": 0.47e9, "per_iteration": 3.168e9}}
+LEARNED_TRAFFIC = {(2, 2048): {"start": 0.083e9, "per_iteration": 0.5957e9},
+                   (3, 256): {"start": 0.471e9, "per_iteration": 3.0543e9}}
 
 
 def reference_full_runs():
